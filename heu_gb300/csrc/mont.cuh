@@ -11,10 +11,11 @@
 // (CIOS) method of Koc, Acar and Kaliski ("Analyzing and comparing Montgomery
 // multiplication algorithms", IEEE Micro 1996) with R = 2^(32*S):
 //   for i in 0..S-1:  T += A*b_i;  m = T_0 * n' mod 2^32;  T += m*N;  T >>= 32
-// Each lane keeps its slice of T plus a small lazy carry word that belongs to
-// the lowest limb of the next lane; carries between lanes are settled once at
-// the end with a ballot-based carry-lookahead (generate/propagate masks added
-// as integers), followed by the conditional subtraction of N.
+// Each lane keeps its slice of T in even and odd columns plus the words above
+// it, which overlap the lowest limbs of the next lane; carries between lanes
+// are settled once at the end with a ballot-based carry-lookahead
+// (generate/propagate masks added as integers), followed by the conditional
+// subtraction of N.
 #pragma once
 #include <cstdint>
 
@@ -263,41 +264,73 @@ __device__ __forceinline__ bool less_than(const uint32_t (&x)[L], const uint32_t
 }
 
 // ---- Montgomery core -------------------------------------------------------
-// T (L limbs) plus lazy carry (c0 + c1*2^32, positioned at limb L) += x * y.
-// Written as plain 64-bit arithmetic: x_j*y + T_j + c never exceeds 2^64 - 1,
-// and the compiler maps each step to one wide multiply-add plus the carry
-// adds, which measured 20% faster on sm_103a than explicit PTX carry chains
-// (mad.lo.cc / madc.hi.cc) for the same rows.
+// The running value T of a multiplication is held in two column arrays of one
+// lane's slice, so that every 32x32->64 product lands on one aligned pair of
+// words and a row is one carry chain of wide multiply-adds per parity:
+//   T = sum Ev[j] 2^(32 j) + sum Od[j] 2^(32 (j+1)) + ov 2^(32 (L+1)) + c1
+// (products x[j]*y of even j go to the pairs of Ev, of odd j to the pairs of
+// Od).  Dropping the lowest limb swaps the two arrays' roles: Od becomes the
+// even array, Ev moved down by two words the odd one, and Ev's word 1, now at
+// position 0, is the pending c1.
+//
+// Bound: the fmaheavy pipe, which runs one wide multiply-add per 4 cycles of
+// a sub-partition.  ptxas joins each mad.lo.cc / madc.hi.cc pair on the same
+// operands into one wide multiply-add with carry in and out, so a product
+// costs that one instruction.  Measured on GB300, chains of products of a
+// 2048-bit key: 4 lanes x 16 limbs 8.79 TMAC/s, 8 lanes x 16 limbs 8.87 TMAC/s against
+// 6.42 and 6.47 of the same rows as 64-bit x*y + T + c steps, which need
+// separate adds for both halves of every product.
+
+// Pending c1 and the product row x * y into columns.
 template <int L>
-__device__ __forceinline__ void row_mac(uint32_t (&T)[L], uint32_t& c0, uint32_t& c1, const uint32_t (&x)[L],
-                                        uint32_t y) {
-  uint64_t c = 0;
+__device__ __forceinline__ void row_mac(uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t& ov, uint32_t c1,
+                                        const uint32_t (&x)[L], uint32_t y) {
+  static_assert(L % 2 == 0, "limbs per lane");
+  Ev[0] = add_cc(Ev[0], c1);  // its carry is worth one word: the first of the odd row
 #pragma unroll
-  for (int j = 0; j < L; ++j) {
-    const uint64_t t = (uint64_t)x[j] * y + T[j] + c;
-    T[j] = (uint32_t)t;
-    c = t >> 32;
+  for (int j = 0; j < L; j += 2) {
+    Od[j] = madc_lo_cc(x[j + 1], y, Od[j]);
+    Od[j + 1] = madc_hi_cc(x[j + 1], y, Od[j + 1]);
   }
-  const uint64_t cc = (uint64_t)c0 + c;
-  c0 = (uint32_t)cc;
-  c1 += (uint32_t)(cc >> 32);
-}
-
-// One CIOS reduction-and-shift step with the multiplier limb already added.
-template <int TPI, int L>
-__device__ __forceinline__ void shift_step(uint32_t (&T)[L], uint32_t& c0, uint32_t& c1, const Group<TPI>& g) {
-  uint32_t x = __shfl_down_sync(kFull, T[0], 1, TPI);
-  x = (g.t == TPI - 1) ? 0u : x;
+  ov = addc(ov, 0u);
+  Ev[0] = mad_lo_cc(x[0], y, Ev[0]);
+  Ev[1] = madc_hi_cc(x[0], y, Ev[1]);
 #pragma unroll
-  for (int k = 0; k < L - 1; ++k) T[k] = T[k + 1];
-  T[L - 1] = add_cc(x, c0);
-  c0 = addc(c1, 0u);
-  c1 = 0u;
+  for (int j = 2; j < L; j += 2) {
+    Ev[j] = madc_lo_cc(x[j], y, Ev[j]);
+    Ev[j + 1] = madc_hi_cc(x[j], y, Ev[j + 1]);
+  }
+  Od[L - 1] = addc_cc(Od[L - 1], 0u);
+  ov = addc(ov, 0u);
 }
 
-// Settle the lazy carries and return the bit above the top limb.
+// One reduction step: m = T_0 * n' makes the group's lowest limb zero, then
+// T >>= 32.  On return Od is the even array and Ev the odd one.
 template <int TPI, int L>
-__device__ __forceinline__ uint32_t settle(uint32_t (&T)[L], uint32_t c0, const Group<TPI>& g) {
+__device__ __forceinline__ void reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t& ov, uint32_t& c1,
+                                            const uint32_t (&n)[L], uint32_t np, const Group<TPI>& g) {
+  const uint32_t m = __shfl_sync(kFull, (Ev[0] + c1) * np, 0, TPI);
+  row_mac<L>(Ev, Od, ov, c1, n, m);
+  uint32_t in = __shfl_down_sync(kFull, Ev[0], 1, TPI);
+  in = (g.t == TPI - 1) ? 0u : in;
+  c1 = Ev[1];
+#pragma unroll
+  for (int j = 0; j + 2 < L; ++j) Ev[j] = Ev[j + 2];
+  Ev[L - 2] = in;
+  Ev[L - 1] = ov;
+  ov = 0u;
+}
+
+// Columns -> limbs: settle the carries inside the lane and between lanes and
+// return the word above the top limb.
+template <int TPI, int L>
+__device__ __forceinline__ uint32_t settle(uint32_t (&T)[L], const uint32_t (&Ev)[L], const uint32_t (&Od)[L],
+                                           uint32_t ov, uint32_t c1, const Group<TPI>& g) {
+  T[0] = add_cc(Ev[0], c1);
+#pragma unroll
+  for (int j = 1; j < L; ++j) T[j] = addc_cc(Ev[j], Od[j - 1]);
+  uint32_t c0 = addc(Od[L - 1], 0u);  // at most a few units: the slice's value is below 4 * 2^(32 L)
+  (void)ov;                           // 0 after a step's shift
   uint32_t cin = __shfl_up_sync(kFull, c0, 1, TPI);
   cin = (g.t == 0) ? 0u : cin;
   const uint32_t topc = __shfl_sync(kFull, c0, TPI - 1, TPI);
@@ -321,24 +354,43 @@ __device__ __forceinline__ uint32_t settle(uint32_t (&T)[L], uint32_t c0, const 
 template <int TPI, int L>
 __device__ __forceinline__ void mont_mul(uint32_t (&r)[L], const uint32_t (&a)[L], const uint32_t (&b)[L],
                                          const uint32_t (&n)[L], uint32_t np, const Group<TPI>& g) {
-  uint32_t T[L];
+  uint32_t E[L], O[L], T[L];
 #pragma unroll
-  for (int j = 0; j < L; ++j) T[j] = 0u;
-  uint32_t c0 = 0u, c1 = 0u;
+  for (int j = 0; j < L; ++j) E[j] = O[j] = 0u;
+  uint32_t ov = 0u, c1 = 0u;
 #pragma unroll 1
   for (int owner = 0; owner < TPI; ++owner) {
 #pragma unroll
-    for (int j = 0; j < L; ++j) {
-      const uint32_t bi = __shfl_sync(kFull, b[j], owner, TPI);
-      uint32_t m = (T[0] + a[0] * bi) * np;
-      m = __shfl_sync(kFull, m, 0, TPI);
-      row_mac<L>(T, c0, c1, a, bi);
-      row_mac<L>(T, c0, c1, n, m);
-      shift_step<TPI, L>(T, c0, c1, g);
+    for (int j = 0; j < L; j += 2) {
+      row_mac<L>(E, O, ov, c1, a, __shfl_sync(kFull, b[j], owner, TPI));
+      c1 = 0u;
+      reduce_step<TPI, L>(E, O, ov, c1, n, np, g);
+      row_mac<L>(O, E, ov, c1, a, __shfl_sync(kFull, b[j + 1], owner, TPI));
+      c1 = 0u;
+      reduce_step<TPI, L>(O, E, ov, c1, n, np, g);
     }
   }
-  const uint32_t top = settle<TPI, L>(T, c0, g);
+  const uint32_t top = settle<TPI, L>(T, E, O, ov, c1, g);
   reduce_once<TPI, L>(r, T, top, n, g);
+}
+
+// The S reduction steps of a single-width T: limbs of T * R^-1 (at most N).
+template <int TPI, int L>
+__device__ __forceinline__ uint32_t redc_steps(uint32_t (&T)[L], const uint32_t (&a)[L], const uint32_t (&n)[L],
+                                               uint32_t np, const Group<TPI>& g) {
+  uint32_t E[L], O[L];
+#pragma unroll
+  for (int j = 0; j < L; ++j) {
+    E[j] = a[j];
+    O[j] = 0u;
+  }
+  uint32_t ov = 0u, c1 = 0u;
+#pragma unroll 1
+  for (int s = 0; s < TPI * L; s += 2) {
+    reduce_step<TPI, L>(E, O, ov, c1, n, np, g);
+    reduce_step<TPI, L>(O, E, ov, c1, n, np, g);
+  }
+  return settle<TPI, L>(T, E, O, ov, c1, g);
 }
 
 // r = a * R^-1 mod N (Montgomery reduction of a single-width a < R).
@@ -346,19 +398,7 @@ template <int TPI, int L>
 __device__ __forceinline__ void mont_redc(uint32_t (&r)[L], const uint32_t (&a)[L], const uint32_t (&n)[L],
                                           uint32_t np, const Group<TPI>& g) {
   uint32_t T[L];
-  copy_slice<L>(T, a);
-  uint32_t c0 = 0u, c1 = 0u;
-#pragma unroll 1
-  for (int owner = 0; owner < TPI; ++owner) {
-#pragma unroll
-    for (int j = 0; j < L; ++j) {
-      uint32_t m = T[0] * np;
-      m = __shfl_sync(kFull, m, 0, TPI);
-      row_mac<L>(T, c0, c1, n, m);
-      shift_step<TPI, L>(T, c0, c1, g);
-    }
-  }
-  const uint32_t top = settle<TPI, L>(T, c0, g);
+  const uint32_t top = redc_steps<TPI, L>(T, a, n, np, g);
   reduce_once<TPI, L>(r, T, top, n, g);
 }
 
@@ -367,19 +407,7 @@ template <int TPI, int L>
 __device__ __forceinline__ void mont_redc_wide(uint32_t (&r)[L], const uint32_t (&lo)[L], const uint32_t (&hi)[L],
                                                const uint32_t (&n)[L], uint32_t np, const Group<TPI>& g) {
   uint32_t T[L];
-  copy_slice<L>(T, lo);
-  uint32_t c0 = 0u, c1 = 0u;
-#pragma unroll 1
-  for (int owner = 0; owner < TPI; ++owner) {
-#pragma unroll
-    for (int j = 0; j < L; ++j) {
-      uint32_t m = T[0] * np;
-      m = __shfl_sync(kFull, m, 0, TPI);
-      row_mac<L>(T, c0, c1, n, m);
-      shift_step<TPI, L>(T, c0, c1, g);
-    }
-  }
-  const uint32_t top = settle<TPI, L>(T, c0, g);  // T <= N here, top == 0
+  const uint32_t top = redc_steps<TPI, L>(T, lo, n, np, g);  // T <= N here, top == 0
   uint32_t s[L];
   const uint32_t c = add_full<TPI, L>(s, T, hi, g);
   reduce_once<TPI, L>(r, s, c + top, n, g);
