@@ -1,127 +1,407 @@
-// CRT decryption kernel (decryptor.cc:32-53): two groups of TP lanes per
-// ciphertext, one per prime; persistent grid, each unit slot owning two
-// odd-power tables in scratch and a hand-off buffer in shared memory; warps
-// take ciphertexts from a launch-wide counter (next_work).
+// CRT decryption (decryptor.cc:32-53) in two kernels:
+//   k_dec_pow   c^(p-1) mod p^2 and c^(q-1) mod q^2 by sliding windows, in two
+//               digits to the base of the prime (sqmod.cuh): the result's
+//               second digit is, up to constants of the key, L_p(c^(p-1));
+//   k_dec_tail  m_p, m_q, their CRT combination, the sign fold and decoding.
+//
+// Bound: the fmaheavy pipe (wide multiply-adds).  A squaring of the exponent's
+// 1,024 at 2048 bits costs 4 H^2 multiply-adds with H = 32 limbs, against
+// 8 H^2 of a Montgomery product modulo p^2, and a chain of a prime's limbs in
+// one lane needs no shuffles but one and reads the prime from the constant
+// bank.  65,536 decryptions on GB300: 206 ms with 64-bit rows modulo p^2, 160 ms
+// with the columns of mont.cuh, 89 ms in two digits (84% of the issue bound of
+// the products it makes).
 #include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <type_traits>
 
 #include "paillier_ops.cuh"
+#include "sqmod.cuh"
 
 namespace hg {
 
-namespace {
-constexpr int kBlock = 128;
-
-// Resident blocks per SM the compiler must fit (register budget).  The
-// 2048-bit throughput layout (4 lanes x 16 limbs per side) is held at 96
-// registers so five blocks fit instead of four: decryption 312 k/s -> 322
-// k/s on 2^20 ciphertexts (the extra warps hide more of the dependent
-// multiply-add latency; six blocks, 80 registers, spill and fall back to
-// 315 k/s).  The 3072-bit layout (8 lanes x 12 limbs) likewise fits five
-// blocks in 94 registers without spilling (a mixed-key stream dominated by
-// 3072-bit decryptions: 428 k -> 433 k ops/s per call).  The other layouts
-// keep the compiler's own budget.
-constexpr int dec_min_blocks(int TP, int LP) { return ((TP == 4 && LP == 16) || (TP == 8 && LP == 12)) ? 5 : 1; }
-}  // namespace
-
 void count_launches(uint64_t n);
 
-template <int TP, int LP>
-__global__ void __launch_bounds__(kBlock, dec_min_blocks(TP, LP)) k_decrypt(KeyConst kc, SecConst sc, const uint32_t* __restrict__ ct,
-                                                    size_t count, int64_t* __restrict__ out_i64,
-                                                    uint8_t* __restrict__ out_ovf, uint32_t* __restrict__ out_mag,
-                                                    uint8_t* __restrict__ out_neg, uint32_t* __restrict__ scratch,
-                                                    uint32_t* err, unsigned long long* ctr, Codec cd) {
-  constexpr int SP = TP * LP;
-  constexpr int UPW = 32 / (2 * TP);  // ciphertexts per warp
-  constexpr int UPB = kBlock / (2 * TP);
-  __shared__ __align__(16) uint32_t ysm[UPB][2 * SP];
-  const Group<TP> g;
-  const int lane = threadIdx.x & 31;
-  const int side = (lane / TP) & 1;
-  const int unit_w = lane / (2 * TP);
-  const int unit_b = threadIdx.x / (2 * TP);
-  const int ntab = 1 << (sc.wd - 1);
-  uint32_t* tb = scratch + (((size_t)blockIdx.x * UPB + unit_b) * 2 + side) * (size_t)ntab * SP + g.t * LP;
-  for (size_t wbase = next_work(ctr, UPW); wbase < count; wbase = next_work(ctr, UPW)) {
-    const size_t inst = wbase + unit_w;
-    const bool active = inst < count;
-    decrypt_one<TP, LP>(kc, sc, ct, active ? inst : count - 1, active, side, tb, ysm[unit_b], out_i64, out_ovf,
-                        out_mag, out_neg, g, err, cd);
+namespace {
+
+// Both primes by value: with one lane per chain the multiply-adds take them
+// as constant-bank operands.
+template <int H>
+struct DecPrimes {
+  uint32_t n[2][H];
+};
+
+// Vector words of a lane's slice in the odd-power table.
+template <int L>
+struct SliceVec {
+  using T = typename std::conditional<L % 4 == 0, uint4, uint2>::type;
+  static constexpr int kN = L % 4 == 0 ? L / 4 : L / 2;
+};
+
+// Odd-power table of a warp: [entry][vector][lane], so every load and store
+// of an entry is one contiguous run of the warp.
+template <int L>
+__device__ __forceinline__ void table_load(uint32_t (&x)[L], const uint32_t* tb, int e, uint32_t lane) {
+  using V = typename SliceVec<L>::T;
+  constexpr int kN = SliceVec<L>::kN, kW = sizeof(V) / 4;
+  const V* p = reinterpret_cast<const V*>(tb) + (size_t)e * kN * 32 + lane;
+#pragma unroll
+  for (int q = 0; q < kN; ++q) {
+    const V v = p[q * 32];
+    x[kW * q] = v.x;
+    x[kW * q + 1] = v.y;
+    if constexpr (kW == 4) {
+      x[kW * q + 2] = v.z;
+      x[kW * q + 3] = v.w;
+    }
   }
 }
 
-template <typename K>
-static int occupancy_blocks(K kernel) {
-  int dev = 0, sms = 0, per = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kBlock, 0);
-  return sms * (per > 0 ? per : 1);
+template <int L>
+__device__ __forceinline__ void table_store(uint32_t* tb, int e, uint32_t lane, const uint32_t (&x)[L]) {
+  using V = typename SliceVec<L>::T;
+  constexpr int kN = SliceVec<L>::kN, kW = sizeof(V) / 4;
+  V* p = reinterpret_cast<V*>(tb) + (size_t)e * kN * 32 + lane;
+#pragma unroll
+  for (int q = 0; q < kN; ++q) {
+    if constexpr (kW == 4)
+      p[q * 32] = make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+    else
+      p[q * 32] = make_uint2(x[2 * q], x[2 * q + 1]);
+  }
 }
 
-int units_per_block_decrypt(int Sp, int variant) {
-  const int tp = (Sp == 32) ? (variant ? 4 : 2) : (Sp == 64) ? (variant ? 8 : 4) : (variant ? 4 : 8);
-  return kBlock / (2 * tp);
+// c < n^2 (decryptor.cc:21-23), over all lanes of the instance.
+template <int TC, int L>
+__device__ __forceinline__ bool raw_below(const uint32_t* __restrict__ c, const uint32_t* __restrict__ N) {
+  constexpr int W = 2 * L;  // limbs per lane: 2 TC lanes hold 4 H
+  const Group<2 * TC> g;
+  const uint32_t* a = c + g.t * W;
+  const uint32_t* b = N + g.t * W;
+  uint32_t borrow = 0u;
+  bool same = true;
+#pragma unroll 4
+  for (int j = 0; j < W; ++j) {
+    const uint64_t d = (uint64_t)a[j] - b[j] - borrow;
+    borrow = (uint32_t)(d >> 63);
+    same = same && a[j] == b[j];
+  }
+  uint32_t out;
+  (void)lookahead<2 * TC>(g, borrow != 0u, same, 0u, out);
+  return out != 0u;
 }
 
-int resident_blocks_decrypt(int Sp, int variant) {
-  int r = 0;
-  [&]() -> cudaError_t {
-    HG_DISPATCH_SPV(Sp, variant, r = occupancy_blocks(k_decrypt<TP, LP>));
-    return cudaSuccess;
-  }();
-  return r;
+// One side of a warp's instances: digit 1 of c^(p-1) mod p^2, to
+// z[(2 i + side) H ..].  The exponent program and its table (2^(wd-1) odd
+// powers, then the square) are as in build_prog.
+template <int TC, int L, class Mod>
+__device__ __forceinline__ void dec_pow_side(const Mod& n, const KeyConst& kc, const SecConst& sc, int side,
+                                             const uint32_t* __restrict__ ct, size_t i, bool active, uint32_t* tb,
+                                             uint32_t* area, uint32_t* __restrict__ z, uint32_t* err,
+                                             const SqLanes<TC, L>& g) {
+  constexpr int H = TC * L;
+  const uint32_t np = sc.np1[side];
+  const uint16_t* prog = sc.prog[side];
+  const int ntab = 1 << (sc.wd - 1);
+  const uint32_t* src = ct + i * (4 * H);
+  if (side == 0) {
+    const bool ok = raw_below<TC, L>(src, kc.N);
+    if (active && !ok && g.lane == g.base) atomicOr(err, kErrCtRange);
+  }
+  uint32_t x[L];
+  sq_from_raw<TC, L, 4 * H>(x, src, n, np, g);
+  table_store<L>(tb, 0, g.lane, x);
+  // one loop over the table's products and the program, so that each kind of
+  // pass is compiled once: step 0 squares into slot ntab, step s < ntab makes
+  // slot s from slot s - 1 and the square, the rest is the program
+  const int steps = ntab + sc.prog_len;
+#pragma unroll 1
+  for (int s = 0; s < steps; ++s) {
+    int e = -1;  // -1: square, else multiply by slot e
+    if (s < ntab) {
+      if (s > 0) e = ntab;
+    } else {
+      const uint16_t op = prog[s - ntab];
+      if (op == kOpNop) break;  // only pads the shorter program
+      if (op != kOpSquare) e = op;
+    }
+    if (s == 1) table_load<L>(x, tb, 0, g.lane);
+    if (s == ntab) table_load<L>(x, tb, sc.start[side], g.lane);
+    sq_stage<TC, L>(area, x, e >= 0, g);
+    if (e < 0) {
+      sq_pass<TC, L, false>(x, x, g.limb(area, 0, 0), (uint32_t)g.c, x, nullptr, n, np, g);
+    } else {
+      uint32_t y0[L];
+      table_load<L>(x, tb, e, g.lane);
+      table_load<L>(y0, tb, e, g.lane - g.c * TC);
+      sq_pass<TC, L, true>(x, x, g.limb(area, 0, 0), 0u, y0, g.limb(area, 1, 0), n, np, g);
+    }
+    if (s < ntab) table_store<L>(tb, s == 0 ? ntab : s, g.lane, x);
+  }
+  sq_redc<TC, L>(x, x, n, np, g);
+  // digit 0 is 1, or a multiple of p where p divides c: such a c decrypts as
+  // it always did, through the value that stands for it
+  uint32_t any = x[0] ^ (g.t == 0 ? 1u : 0u);
+#pragma unroll
+  for (int j = 1; j < L; ++j) any |= x[j];
+  const uint32_t mask = (1u << TC) - 1u;
+  const bool zero = ((__ballot_sync(kFull, any != 0u) >> g.base) & mask) != 0u;
+  if (zero) load_slice<L>(x, sc.vz[side] + g.t * L);
+  if (active && g.c == 1) store_slice<L>(z + (2 * i + side) * H + g.t * L, x);
 }
 
-// Batches up to one wave of the latency layout (a half warp per CRT side,
-// one ciphertext per warp), and at most 12 per SM, run in that layout.
-static size_t latency_wave_decrypt(int Sp) {
-  static size_t cache[3] = {0, 0, 0};
-  const int slot = Sp == 32 ? 0 : Sp == 64 ? 1 : 2;
-  if (cache[slot] == 0) {
-    size_t v = 0;
+// Resident warps per SM that the compiler must fit, one warp per block.  The
+// multiply-add pipe is 91% busy at 8 warps, so the one-lane layouts take the
+// registers they need: 65,536 decryptions of 2048 bits took 89.8 ms at 10 warps
+// against 92.0 at 12 and 100.7 at 16, whose two-row pass spills.
+constexpr int dec_min_blocks(int L) { return L == 48 ? 8 : L == 32 ? 10 : L == 24 ? 12 : L == 16 ? 16 : L == 12 ? 18 : 20; }
+
+// One warp per block: warps take (side, group of instances) items from the
+// launch's counter, all first sides before the second ones.
+template <int TC, int L>
+__global__ void __launch_bounds__(32, dec_min_blocks(L))
+    k_dec_pow(const __grid_constant__ DecPrimes<TC * L> primes, const __grid_constant__ KeyConst kc,
+              const __grid_constant__ SecConst sc, const uint32_t* __restrict__ ct, size_t count,
+              uint32_t* __restrict__ scratch, uint32_t* __restrict__ z, uint32_t* err, unsigned long long* ctr) {
+  using G = SqLanes<TC, L>;
+  __shared__ uint32_t area[G::kWords];
+  const G g;
+  const size_t slots = ((size_t)1 << (sc.wd - 1)) + 1;
+  uint32_t* tb = scratch + (size_t)blockIdx.x * slots * 32 * L;
+  const size_t groups = (count + G::IPW - 1) / G::IPW;
+  for (size_t item = next_work(ctr, 1); item < 2 * groups; item = next_work(ctr, 1)) {
+    const int side = item < groups ? 0 : 1;
+    const size_t inst = (item - (side ? groups : 0)) * G::IPW + g.iw;
+    const bool active = inst < count;
+    const size_t i = active ? inst : count - 1;
+    if constexpr (TC == 1) {
+      if (side == 0)
+        dec_pow_side<TC, L>(primes.n[0], kc, sc, 0, ct, i, active, tb, area, z, err, g);
+      else
+        dec_pow_side<TC, L>(primes.n[1], kc, sc, 1, ct, i, active, tb, area, z, err, g);
+    } else {
+      uint32_t n[L];
+      load_slice<L>(n, sc.P[side] + g.t * L);
+      dec_pow_side<TC, L>(n, kc, sc, side, ct, i, active, tb, area, z, err, g);
+    }
+  }
+}
+
+// m_p = z_p c1_p + c2_p mod p, the same for q, then the CRT combination
+//   h = (m_q - m_p) p^-1 mod q, m = m_p + p h
+// and the sign fold m > n/2 => m - n (decryptor.cc:49-52).  8 lanes per
+// ciphertext; under 1% of the decryption.
+template <int LT>
+__global__ void __launch_bounds__(128) k_dec_tail(const __grid_constant__ KeyConst kc,
+                                                  const __grid_constant__ SecConst sc,
+                                                  const uint32_t* __restrict__ z, size_t count,
+                                                  int64_t* __restrict__ out_i64, uint8_t* __restrict__ out_ovf,
+                                                  uint32_t* __restrict__ out_mag, uint8_t* __restrict__ out_neg,
+                                                  const __grid_constant__ Codec cd, size_t first) {
+  constexpr int TP = 8, H = TP * LT, W = 2 * LT;
+  __shared__ __align__(16) uint32_t mms[128 / TP][2 * H];
+  const Group<TP> g;
+  const size_t inst = ((size_t)blockIdx.x * 128 + threadIdx.x) / TP;
+  const bool active = inst < count;
+  const size_t u = active ? inst : count - 1;
+  const size_t i = first + u;
+  uint32_t* mm = mms[threadIdx.x / TP];
+  uint32_t P[LT], Q[LT], a[LT], b[LT], mp[LT], mq[LT];
+  load_slice<LT>(P, sc.P[0] + g.t * LT);
+  load_slice<LT>(Q, sc.P[1] + g.t * LT);
+  load_slice<LT>(a, z + (2 * u) * H + g.t * LT);
+  load_slice<LT>(b, sc.c1[0] + g.t * LT);
+  mont_mul<TP, LT>(mp, a, b, P, sc.np1[0], g);
+  load_slice<LT>(b, sc.c2[0] + g.t * LT);
+  mod_add<TP, LT>(mp, mp, b, P, g);
+  load_slice<LT>(a, z + (2 * u + 1) * H + g.t * LT);
+  load_slice<LT>(b, sc.c1[1] + g.t * LT);
+  mont_mul<TP, LT>(mq, a, b, Q, sc.np1[1], g);
+  load_slice<LT>(b, sc.c2[1] + g.t * LT);
+  mod_add<TP, LT>(mq, mq, b, Q, g);
+  // m_p mod q (p < 2q), then h
+  reduce_once<TP, LT>(a, mp, 0u, Q, g);
+  mod_sub<TP, LT>(mq, mq, a, Q, g);
+  load_slice<LT>(b, sc.pinvqR + g.t * LT);
+  mont_mul<TP, LT>(mq, mq, b, Q, sc.np1[1], g);
+  // m = m_p + p h: rows of p, the lowest limb leaves in every step
+  {
+    uint32_t E[LT], O[LT], T[LT], ov = 0u, c1 = 0u;
+#pragma unroll
+    for (int j = 0; j < LT; ++j) {
+      E[j] = mp[j];
+      O[j] = 0u;
+    }
+#pragma unroll 1
+    for (int owner = 0; owner < TP; ++owner) {
+#pragma unroll
+      for (int j = 0; j < LT; j += 2) {
+        row_mac<LT>(E, O, ov, c1, P, __shfl_sync(kFull, mq[j], owner, TP));
+        if (g.t == 0) mm[owner * LT + j] = E[0];
+        shift_limb<TP, LT>(E, ov, c1, g);
+        row_mac<LT>(O, E, ov, c1, P, __shfl_sync(kFull, mq[j + 1], owner, TP));
+        if (g.t == 0) mm[owner * LT + j + 1] = O[0];
+        shift_limb<TP, LT>(O, ov, c1, g);
+      }
+    }
+    (void)settle<TP, LT>(T, E, O, ov, c1, g);
+    store_slice<LT>(mm + H + g.t * LT, T);
+  }
+  __syncwarp();
+  uint32_t M[W], X[W], D[W];
+  load_slice<W>(M, mm + g.t * W);
+  load_slice<W>(X, kc.nhalf + g.t * W);
+  const bool gt = sub_full<TP, W>(D, X, M, g) != 0u;
+  load_slice<W>(X, kc.n + g.t * W);
+  (void)sub_full<TP, W>(D, X, M, g);
+  select_slice<W>(M, gt, D, M);
+  __syncwarp();
+  store_slice<W>(mm + g.t * W, M);
+  __syncwarp();
+  if (cd.kind != kCodecNone) {
+    if (active && g.t == 0) decode_plain<2 * H>(cd, mm, gt, i, out_i64, out_ovf);
+    return;
+  }
+  if (out_mag) {
+    if (active) store_slice<W>(out_mag + i * (2 * H) + g.t * W, M);
+    if (active && g.t == 0) out_neg[i] = gt ? 1 : 0;
+  }
+  if (out_i64) {
+    uint32_t high = 0u;
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+      if (g.t != 0 || j >= 2) high |= M[j];
+    const uint32_t B = __ballot_sync(kFull, high != 0u);
+    bool fits = ((B >> g.base) & 0xffu) == 0u;
+    if (active && g.t == 0) {
+      const uint64_t mag = (uint64_t)M[0] | ((uint64_t)M[1] << 32);
+      fits = fits && (gt ? mag <= (1ull << 63) : mag < (1ull << 63));
+      out_i64[i] = (int64_t)(gt ? (uint64_t)0 - mag : mag);
+      if (out_ovf) out_ovf[i] = fits ? 0 : 1;
+    }
+  }
+}
+
+// Layouts by (limbs of a prime, log2 of the lanes per chain).
+#define HG_DISPATCH_DEC(H, LOGTC, ...)                                          \
+  switch ((H) * 8 + (LOGTC)) {                                                  \
+    case 128: { constexpr int TC = 1, L = 16; __VA_ARGS__; } break;             \
+    case 129: { constexpr int TC = 2, L = 8; __VA_ARGS__; } break;              \
+    case 130: { constexpr int TC = 4, L = 4; __VA_ARGS__; } break;              \
+    case 131: { constexpr int TC = 8, L = 2; __VA_ARGS__; } break;              \
+    case 256: { constexpr int TC = 1, L = 32; __VA_ARGS__; } break;             \
+    case 257: { constexpr int TC = 2, L = 16; __VA_ARGS__; } break;             \
+    case 258: { constexpr int TC = 4, L = 8; __VA_ARGS__; } break;              \
+    case 259: { constexpr int TC = 8, L = 4; __VA_ARGS__; } break;              \
+    case 260: { constexpr int TC = 16, L = 2; __VA_ARGS__; } break;             \
+    case 384: { constexpr int TC = 1, L = 48; __VA_ARGS__; } break;             \
+    case 385: { constexpr int TC = 2, L = 24; __VA_ARGS__; } break;             \
+    case 386: { constexpr int TC = 4, L = 12; __VA_ARGS__; } break;             \
+    case 387: { constexpr int TC = 8, L = 6; __VA_ARGS__; } break;              \
+    default: return cudaErrorInvalidValue;                                      \
+  }
+
+int layouts(int H) { return H == 32 ? 5 : 4; }
+
+// Resident warps of the whole device in a layout, cached per device-wide kernel.
+int resident_warps(int H, int logtc) {
+  static std::atomic<int> cache[3][5];
+  std::atomic<int>& slot = cache[H == 16 ? 0 : H == 32 ? 1 : 2][logtc];
+  int v = slot.load(std::memory_order_relaxed);
+  if (v == 0) {
+    int dev = 0, sms = 0, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     [&]() -> cudaError_t {
-      HG_DISPATCH_SPL(Sp, v = (size_t)occupancy_blocks(k_decrypt<TP, LP>) * (kBlock / 32));
-      int dev = 0, sms = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-      // at most 12 ciphertexts per SM (4096 took 18.3 ms in this layout
-      // against 16.1 ms in the throughput layout on GB300, one 4.2 ms
-      // against 10.2 ms)
-      v = std::min(v, (size_t)12 * (size_t)sms);
+      HG_DISPATCH_DEC(H, logtc, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_dec_pow<TC, L>, 32, 0));
       return cudaSuccess;
     }();
-    cache[slot] = v;
+    v = sms * std::max(per, 1);
+    slot.store(v, std::memory_order_relaxed);
   }
-  return cache[slot];
+  return v;
 }
 
-cudaError_t launch_decrypt(int Sp, const KeyConst& kc, const SecConst& sc, const uint32_t* ct, size_t count,
-                           int64_t* out_i64, uint8_t* out_ovf, uint32_t* out_mag, uint8_t* out_neg,
-                           uint32_t* scratch, uint32_t* err, int grid, unsigned long long* ctr, cudaStream_t st,
-                           const Codec& cd) {
-  if (count == 0) return cudaSuccess;
-  const cudaError_t e = cudaMemsetAsync(ctr, 0, sizeof(*ctr), st);
-  if (e != cudaSuccess) return e;
-  // the latency layout's unit slots must fit the scratch sized for `grid`
-  // blocks of the throughput layout
-  const size_t lat_blocks = (count + kBlock / 32 - 1) / (kBlock / 32);
-  if (count <= latency_wave_decrypt(Sp) &&
-      lat_blocks * (kBlock / 32) <= (size_t)grid * units_per_block_decrypt(Sp, sc.variant)) {
-    HG_DISPATCH_SPL(Sp, k_decrypt<TP, LP><<<(unsigned)lat_blocks, kBlock, 0, st>>>(
-                            kc, sc, ct, count, out_i64, out_ovf, out_mag, out_neg, scratch, err, ctr, cd));
-    count_launches(1);
-    return cudaGetLastError();
-  }
-  HG_DISPATCH_SPV(Sp, sc.variant, {
-    const size_t upb = kBlock / (2 * TP);
-    const unsigned need = (unsigned)((count + upb - 1) / upb);
-    const unsigned gb = (unsigned)std::min((size_t)need, (size_t)grid);
-    k_decrypt<TP, LP><<<gb, kBlock, 0, st>>>(kc, sc, ct, count, out_i64, out_ovf, out_mag, out_neg, scratch, err,
-                                             ctr, cd);
-  });
-  count_launches(1);
-  return cudaGetLastError();
+// Time of one item (ms) when every scheduler holds `warps` warps of a layout,
+// as measured on GB300 with the default windows: more lanes per chain shorten
+// the chain of dependent steps but spend more shuffles per limb, so few
+// ciphertexts run fastest in the widest layout and many in the narrowest.
+// 2048 bits: 8 ciphertexts take 1.97 ms with 16 lanes a chain against 10.7 ms
+// with one, 2,432 take 4.1 ms with 4 lanes (5.2 with 8, 6.0 with 2), 131,072
+// take 169 ms with one lane against 180 with two.
+double item_cost(int H, int logtc, double warps) {
+  static const double lat[3][5] = {{1.32, 0.95, 0.78, 0.62, 0}, {10.2, 5.7, 2.9, 2.14, 1.96}, {29, 17.5, 8.6, 5.2, 0}};
+  static const double thr[3][5] = {{0.85, 0.53, 0.31, 0.2, 0}, {6.5, 3.4, 1.98, 1.27, 0.83}, {20.3, 11.1, 5.95, 3.4, 0}};
+  const int r = H == 16 ? 0 : H == 32 ? 1 : 2;
+  return std::max(lat[r][logtc], thr[r][logtc] * warps);
 }
+
+constexpr size_t kHandoffBytes = (size_t)128 << 20;  // digits between the two kernels, at most
+
+}  // namespace
+
+DecryptPlan decrypt_plan(int Sp, const SecConst& sc, size_t count) {
+  const int H = Sp / 2;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const double scheds = 4.0 * std::max(sms, 1);
+  DecryptPlan pl;
+  pl.chunk = std::min(count, kHandoffBytes / ((size_t)2 * H * 4));
+  double best = 1e300;
+  for (int l = sc.variant ? 1 : 0; l < layouts(H); ++l) {
+    const size_t ipw = (size_t)16 >> l;
+    const size_t items = 2 * ((pl.chunk + ipw - 1) / ipw);
+    const size_t cap = (size_t)resident_warps(H, l);
+    const size_t rounds = (items + cap - 1) / cap;
+    const size_t warps = (items + rounds - 1) / rounds;  // every warp the same number of items
+    const double per = std::ceil((double)warps / scheds);
+    const double cost = (double)rounds * item_cost(H, l, per);
+    if (cost < best) {
+      best = cost;
+      pl.logtc = l;
+      pl.warps = (int)warps;
+    }
+  }
+  const size_t slots = ((size_t)1 << (sc.wd - 1)) + 1;
+  pl.table_words = (size_t)pl.warps * slots * 32 * (size_t)(H >> pl.logtc);
+  pl.handoff_words = pl.chunk * 2 * (size_t)H;
+  return pl;
+}
+
+cudaError_t launch_decrypt(int Sp, const KeyConst& kc, const SecConst& sc, const uint32_t* primes,
+                           const DecryptPlan& pl, const uint32_t* ct, size_t count, int64_t* out_i64,
+                           uint8_t* out_ovf, uint32_t* out_mag, uint8_t* out_neg, uint32_t* scratch, uint32_t* err,
+                           unsigned long long* ctr, cudaStream_t st, const Codec& cd) {
+  const int H = Sp / 2;
+  uint32_t* z = scratch + pl.table_words;
+  for (size_t off = 0; off < count; off += pl.chunk) {
+    const size_t n = std::min(pl.chunk, count - off);
+    cudaError_t e = cudaMemsetAsync(ctr, 0, sizeof(*ctr), st);
+    if (e != cudaSuccess) return e;
+    HG_DISPATCH_DEC(H, pl.logtc, {
+      DecPrimes<TC * L> pr;
+      std::copy(primes, primes + 2 * TC * L, &pr.n[0][0]);
+      const size_t items = 2 * ((n + SqLanes<TC, L>::IPW - 1) / SqLanes<TC, L>::IPW);
+      k_dec_pow<TC, L><<<(unsigned)std::min(items, (size_t)pl.warps), 32, 0, st>>>(pr, kc, sc, ct + off * 4 * H, n,
+                                                                                  scratch, z, err, ctr);
+    });
+    count_launches(1);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    const unsigned blocks = (unsigned)((n + 15) / 16);
+    switch (H) {
+      case 16: k_dec_tail<2><<<blocks, 128, 0, st>>>(kc, sc, z, n, out_i64, out_ovf, out_mag, out_neg, cd, off); break;
+      case 32: k_dec_tail<4><<<blocks, 128, 0, st>>>(kc, sc, z, n, out_i64, out_ovf, out_mag, out_neg, cd, off); break;
+      case 48: k_dec_tail<6><<<blocks, 128, 0, st>>>(kc, sc, z, n, out_i64, out_ovf, out_mag, out_neg, cd, off); break;
+      default: return cudaErrorInvalidValue;
+    }
+    count_launches(1);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+size_t decrypt_wave(int Sp) { return (size_t)resident_warps(Sp / 2, 0) * 16 / 2; }
 
 }  // namespace hg

@@ -177,7 +177,8 @@ struct KeyRec {
   DevBuf consts, sconsts, table, progs;
   hg::KeyConst kc{};
   hg::SecConst sc{};
-  int grid_mul = 0, grid_dec = 0;
+  int grid_mul = 0;
+  std::vector<uint32_t> primes;  // p, q (H limbs each)
   int grid_mul_bn = 0;  // persistent grid of the multi-limb scalar Mul (set on first use)
   int wm = 4;  // scalar-mul window
   // Okamoto-Uchiyama keys (scheme 1): kc is over n with the H table; kcG /
@@ -484,15 +485,21 @@ void core_encrypt_encoded(KeyRec& k, Work& w, const void* values, const uint32_t
              "encrypt launch");
 }
 
+// CRT decryption into any of the output forms.
+void decrypt_crt(KeyRec& k, Work& w, const uint32_t* ct, int64_t* m, uint8_t* ovf, uint32_t* mag, uint8_t* neg,
+                 size_t count, const hg::Codec& cd) {
+  if (!k.secret) fail(HG_ERR_NO_SECRET, "key has no secret part");
+  if (count == 0) return;
+  const hg::DecryptPlan pl = hg::decrypt_plan(k.Sp, k.sc, count);
+  uint32_t* scratch = w.scratch.ensure<uint32_t>((pl.table_words + pl.handoff_words) * 4);
+  cuda_check(hg::launch_decrypt(k.Sp, k.kc, k.sc, k.primes.data(), pl, ct, count, m, ovf, mag, neg, scratch, w.errp(),
+                                w.ctrp(), w.stream, cd),
+             "decrypt launch");
+}
+
 void core_decrypt_decoded(KeyRec& k, Work& w, const uint32_t* ct, void* out, uint8_t* ovf, size_t count,
                           const hg::Codec& cd) {
-  if (!k.secret) fail(HG_ERR_NO_SECRET, "key has no secret part");
-  const size_t ntab = (size_t)1 << (k.sc.wd - 1);
-  const size_t units = (size_t)k.grid_dec * hg::units_per_block_decrypt(k.Sp, k.sc.variant);
-  uint32_t* scratch = w.scratch.ensure<uint32_t>(units * 2 * ntab * k.Sp * 4);
-  cuda_check(hg::launch_decrypt(k.Sp, k.kc, k.sc, ct, count, static_cast<int64_t*>(out), ovf, nullptr, nullptr,
-                                scratch, w.errp(), k.grid_dec, w.ctrp(), w.stream, cd),
-             "decrypt launch");
+  decrypt_crt(k, w, ct, static_cast<int64_t*>(out), ovf, nullptr, nullptr, count, cd);
 }
 
 // Add(ct, pt) / Sub(ct, pt) with int64 plaintexts, per scheme.
@@ -506,8 +513,8 @@ void core_add_plain(KeyRec& k, Work& w, const uint32_t* a, const int64_t* p, int
 
 void core_decrypt(KeyRec& k, Work& w, const uint32_t* ct, int64_t* m, uint8_t* ovf, uint32_t* mag, uint8_t* neg,
                   size_t count) {
-  if (!k.secret) fail(HG_ERR_NO_SECRET, "key has no secret part");
   if (k.scheme == 1) {
+    if (!k.secret) fail(HG_ERR_NO_SECRET, "key has no secret part");
     const size_t ntab = (size_t)1 << (k.oc.wd - 1);
     const size_t units = (size_t)k.grid_oudec * k.upb_oudec;
     uint32_t* scratch = w.scratch.ensure<uint32_t>(units * ntab * k.oc.Sp * 4);
@@ -516,12 +523,7 @@ void core_decrypt(KeyRec& k, Work& w, const uint32_t* ct, int64_t* m, uint8_t* o
                "OU decrypt launch");
     return;
   }
-  const size_t ntab = (size_t)1 << (k.sc.wd - 1);
-  const size_t units = (size_t)k.grid_dec * hg::units_per_block_decrypt(k.Sp, k.sc.variant);
-  uint32_t* scratch = w.scratch.ensure<uint32_t>(units * 2 * ntab * k.Sp * 4);
-  cuda_check(hg::launch_decrypt(k.Sp, k.kc, k.sc, ct, count, m, ovf, mag, neg, scratch, w.errp(), k.grid_dec,
-                                w.ctrp(), w.stream),
-             "decrypt launch");
+  decrypt_crt(k, w, ct, m, ovf, mag, neg, count, hg::Codec{});
 }
 
 // out[i] = in[i]^-1 where sel == nullptr or sel[i] < 0, else in[i].
@@ -920,17 +922,12 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
     k->secret = true;
     const BN p2 = k->p * k->p, q2 = k->q * k->q;
     const BN R1h = BN(1).shl(32 * (size_t)H);
-    auto hfun = [&](const BN& pr, const BN& pr2) {
-      // secret_key.cc:33-42: h = L((n+1)^(pr-1) mod pr^2)^-1 mod pr
-      const BN g = k->n + BN(1);
-      BN hv = hg::HostMont(pr2).pow(g, pr - BN(1));
-      hv = (hv - BN(1)) / pr;
-      return BN::invmod(hv, pr);
-    };
-    const BN hp = hfun(k->p, p2), hq = hfun(k->q, q2);
+    // secret_key.cc:33-42: h = L((n+1)^(pr-1) mod pr^2)^-1 mod pr; with n = 0
+    // mod pr the power is 1 + (pr-1) n, so L is -n/pr mod pr
+    const BN hp = BN::invmod(k->p - k->q % k->p, k->p), hq = BN::invmod(k->q - k->p % k->q, k->q);
     const BN pinvq = BN::invmod(k->p, k->q);
-    // p2 q2 (Sp) | p q hR_p hR_q inv2_p inv2_q pinvqR (H)
-    std::vector<uint32_t> hs2(2 * (size_t)Sp + 7 * (size_t)H);
+    // p2 q2 (Sp) | p q hR_p hR_q inv2_p inv2_q pinvqR c1_p c1_q c2_p c2_q vz_p vz_q (H)
+    std::vector<uint32_t> hs2(2 * (size_t)Sp + 13 * (size_t)H);
     auto put2 = [&](size_t at, const BN& v, size_t limbs) { v.to_limbs(hs2.data() + at, limbs); };
     put2(0, p2, Sp);
     put2(Sp, q2, Sp);
@@ -939,9 +936,25 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
     put2(o + H, k->q, H);
     put2(o + 2 * H, (hp * R1h) % k->p, H);
     put2(o + 3 * H, (hq * R1h) % k->q, H);
-    put2(o + 4 * H, BN::invmod(k->p, R1h), H);
-    put2(o + 5 * H, BN::invmod(k->q, R1h), H);
+    const BN inv2[2] = {BN::invmod(k->p, R1h), BN::invmod(k->q, R1h)};
+    put2(o + 4 * H, inv2[0], H);
+    put2(o + 5 * H, inv2[1], H);
     put2(o + 6 * H, (pinvq * R1h) % k->q, H);
+    for (int sd = 0; sd < 2; ++sd) {
+      const BN &pr = sd ? k->q : k->p, &pr2 = sd ? q2 : p2, &h = sd ? hq : hp;
+      auto neg = [&](const BN& v) { return v.is_zero() ? v : pr - v; };  // v < pr
+      // 2^-64 is what the input conversion leaves in the ciphertext's digits:
+      // its power is 1 + d pr with d = -64 (2^(pr-1) - 1) / pr
+      const BN l2 = (hg::HostMont(pr2).pow2(pr - BN(1)) - BN(1)) / pr;
+      const BN d = neg((l2 * BN(64)) % pr);
+      const BN lz = (R1h - inv2[sd]) % pr;
+      put2(o + (7 + sd) * H, neg((h * R1h) % pr), H);
+      put2(o + (9 + sd) * H, neg((d * h) % pr), H);
+      put2(o + (11 + sd) * H, neg((lz + d) % pr), H);
+    }
+    k->primes.assign(2 * (size_t)H, 0u);
+    k->p.to_limbs(k->primes.data(), H);
+    k->q.to_limbs(k->primes.data() + H, H);
     uint32_t* ds = k->sconsts.ensure<uint32_t>(hs2.size() * 4);
     cuda_check(cudaMemcpy(ds, hs2.data(), hs2.size() * 4, cudaMemcpyHostToDevice), "upload secret consts");
     auto& sc = k->sc;
@@ -955,11 +968,17 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
     sc.inv2[0] = ds + o + 4 * H;
     sc.inv2[1] = ds + o + 5 * H;
     sc.pinvqR = ds + o + 6 * H;
+    for (int sd = 0; sd < 2; ++sd) {
+      sc.c1[sd] = ds + o + (7 + sd) * H;
+      sc.c2[sd] = ds + o + (9 + sd) * H;
+      sc.vz[sd] = ds + o + (11 + sd) * H;
+    }
     sc.np2[0] = neg_inv32(p2.d[0]);
     sc.np2[1] = neg_inv32(q2.d[0]);
     sc.np1[0] = neg_inv32(k->p.d[0]);
     sc.np1[1] = neg_inv32(k->q.d[0]);
-    sc.wd = 5;
+    // fewest products: (k/2) / (w + 1) windows and 2^(w-1) odd powers
+    sc.wd = key_bits > 1024 ? 6 : 5;
     std::vector<uint16_t> pp, pq;
     build_prog(k->p - BN(1), sc.wd, &sc.start[0], &pp);
     build_prog(k->q - BN(1), sc.wd, &sc.start[1], &pq);
@@ -975,7 +994,6 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
     sc.prog[0] = dp;
     sc.prog[1] = dp + len;
     sc.variant = 0;
-    k->grid_dec = hg::resident_blocks_decrypt(Sp, 0);
   }
   std::lock_guard<std::mutex> lk(ctx->mu);
   const int id = ctx->next_key++;
@@ -2237,7 +2255,6 @@ static void apply_config(KeyRec& k, const hg_key_config& c) {
       k.sc.wd = c.dec_window;
     }
     k.sc.variant = c.dec_variant;
-    k.grid_dec = hg::resident_blocks_decrypt(k.Sp, c.dec_variant);
   }
 }
 
@@ -2561,7 +2578,7 @@ int hg_autotune(hg_ctx* ctx, int key_id, size_t calib, hg_key_config* best, doub
       core_encrypt(*k, w, hg::EncMode::kEncrypt, dm, nullptr, nullptr, dr, nullptr, dct, n);
       // enough ciphertexts for several waves of the widest layout, else the
       // layout with more lanes per ciphertext wins on a half-empty GPU
-      const size_t wave = (size_t)hg::resident_blocks_decrypt(k->Sp, 0) * hg::units_per_block_decrypt(k->Sp, 0);
+      const size_t wave = hg::decrypt_wave(k->Sp);
       const size_t nd = std::min(n, std::max<size_t>(n / 2, 4 * wave));
       double best_d = 1e300;
       for (int dv = 0; dv < 2; ++dv)

@@ -490,6 +490,17 @@ class HostMont {
     }
     return from(r);
   }
+  // 2^e mod m: squarings, and a doubling where the exponent's bit is set
+  BN pow2(const BN& e) const {
+    std::vector<uint32_t> r = one();
+    for (size_t i = e.bitlen(); i-- > 0;) {
+      r = mul(r, r);
+      if (!e.bit(i)) continue;
+      const BN v = BN::from_limbs(r.data(), s_).shl(1);
+      r = (v >= m_ ? v - m_ : v).limbs(s_);
+    }
+    return from(r);
+  }
   std::vector<uint32_t> pad(const BN& a) const { return a.limbs(s_); }
 
  private:

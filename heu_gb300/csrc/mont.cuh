@@ -304,13 +304,10 @@ __device__ __forceinline__ void row_mac(uint32_t (&Ev)[L], uint32_t (&Od)[L], ui
   ov = addc(ov, 0u);
 }
 
-// One reduction step: m = T_0 * n' makes the group's lowest limb zero, then
-// T >>= 32.  On return Od is the even array and Ev the odd one.
+// T >>= 32 in every lane of the group (the lowest limb is dropped; in the
+// other lanes it moves to the lane below).  The roles of the arrays swap.
 template <int TPI, int L>
-__device__ __forceinline__ void reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t& ov, uint32_t& c1,
-                                            const uint32_t (&n)[L], uint32_t np, const Group<TPI>& g) {
-  const uint32_t m = __shfl_sync(kFull, (Ev[0] + c1) * np, 0, TPI);
-  row_mac<L>(Ev, Od, ov, c1, n, m);
+__device__ __forceinline__ void shift_limb(uint32_t (&Ev)[L], uint32_t& ov, uint32_t& c1, const Group<TPI>& g) {
   uint32_t in = __shfl_down_sync(kFull, Ev[0], 1, TPI);
   in = (g.t == TPI - 1) ? 0u : in;
   c1 = Ev[1];
@@ -319,6 +316,16 @@ __device__ __forceinline__ void reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)[L]
   Ev[L - 2] = in;
   Ev[L - 1] = ov;
   ov = 0u;
+}
+
+// One reduction step: m = T_0 * n' makes the group's lowest limb zero, then
+// T >>= 32.  On return Od is the even array and Ev the odd one.
+template <int TPI, int L>
+__device__ __forceinline__ void reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t& ov, uint32_t& c1,
+                                            const uint32_t (&n)[L], uint32_t np, const Group<TPI>& g) {
+  const uint32_t m = __shfl_sync(kFull, (Ev[0] + c1) * np, 0, TPI);
+  row_mac<L>(Ev, Od, ov, c1, n, m);
+  shift_limb<TPI, L>(Ev, ov, c1, g);
 }
 
 // Columns -> limbs: settle the carries inside the lane and between lanes and

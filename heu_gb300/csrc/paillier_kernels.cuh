@@ -42,6 +42,12 @@ struct SecConst {
   const uint32_t* hR[2];    // hp*R1 mod p, hq*R1 mod q    (Sp/2 limbs), R1 = 2^(16*Sp)
   const uint32_t* inv2[2];  // p^-1, q^-1 mod 2^(16*Sp)    (Sp/2 limbs)
   const uint32_t* pinvqR;   // (p^-1 mod q)*R1 mod q       (Sp/2 limbs)
+  // two-digit decryption (decrypt_kernels.cu): with C^(p-1) = 1 + L p mod p^2,
+  // delta = 2^-64 (what its input conversion leaves in C) and delta^(p-1) =
+  // 1 + d p, digit 1 of the result is z = -(L + d): m_p = L hp = z*c1*R1^-1 + c2
+  const uint32_t* c1[2];    // -hp*R1 mod p, -hq*R1 mod q  (Sp/2 limbs)
+  const uint32_t* c2[2];    // -d*hp mod p, the same for q (Sp/2 limbs)
+  const uint32_t* vz[2];    // z that stands for C = 0 mod p: L = -p^-1 mod R1
   const uint16_t* prog[2];  // exponent programs for p-1, q-1
   uint32_t np2[2];          // -(p^2)^-1, -(q^2)^-1 mod 2^32
   uint32_t np1[2];          // -p^-1, -q^-1 mod 2^32
@@ -115,10 +121,20 @@ int resident_blocks_mul_bn(int S);
 cudaError_t launch_sel_from_neg(const uint8_t* neg, int64_t* sel, size_t count, cudaStream_t st);
 // With cd.kind != kCodecNone out_i64 receives the decoded values (int64 or
 // double, per cd.kind) and cd.out1 the second slot of batch kinds.
-cudaError_t launch_decrypt(int Sp, const KeyConst& kc, const SecConst& sc, const uint32_t* ct, size_t count,
-                           int64_t* out_i64, uint8_t* out_ovf, uint32_t* out_mag, uint8_t* out_neg,
-                           uint32_t* scratch, uint32_t* err, int grid, unsigned long long* ctr, cudaStream_t st,
-                           const Codec& cd = Codec{});
+// `primes`: p and q on the host (Sp/2 limbs each); `scratch` holds
+// decrypt_plan's table_words + handoff_words limbs.
+struct DecryptPlan {
+  int logtc = 0;         // log2 of the lanes per chain
+  int warps = 0;         // warps of the exponentiation launch
+  size_t chunk = 0;      // ciphertexts per pair of launches
+  size_t table_words = 0, handoff_words = 0;
+};
+DecryptPlan decrypt_plan(int Sp, const SecConst& sc, size_t count);
+cudaError_t launch_decrypt(int Sp, const KeyConst& kc, const SecConst& sc, const uint32_t* primes,
+                           const DecryptPlan& pl, const uint32_t* ct, size_t count, int64_t* out_i64,
+                           uint8_t* out_ovf, uint32_t* out_mag, uint8_t* out_neg, uint32_t* scratch, uint32_t* err,
+                           unsigned long long* ctr, cudaStream_t st, const Codec& cd = Codec{});
+size_t decrypt_wave(int Sp);  // ciphertexts of one full wave of the widest layout
 // OU decryption over S-limb ciphertexts with Sp-limb p^2 arithmetic
 // (S, Sp) in {(64, 32), (128, 64), (128, 96)}.
 cudaError_t launch_ou_decrypt(int S, const KeyConst& kc, const OuConst& oc, const uint32_t* ct, size_t count,
@@ -194,9 +210,7 @@ size_t subset_table_bytes_per_row(int S, int K);
 
 // Occupancy-derived grid sizes (blocks) for the persistent kernels.
 int resident_blocks_mul(int S, int variant);
-int resident_blocks_decrypt(int Sp, int variant);
 int instances_per_block(int S, int variant);
-int units_per_block_decrypt(int Sp, int variant);
 
 bool supported_limbs(int S);
 uint64_t launch_count();  // kernels launched by this process so far

@@ -129,6 +129,16 @@ __device__ __forceinline__ void sq_settle(uint32_t (&x)[L], const uint32_t (&Ev)
   }
 }
 
+// Steps per round of a pass.  Between rounds the columns return to their
+// registers (about two moves per limb, some of them on the multiply-add pipe),
+// so more steps cost less, until the passes of a kernel leave the instruction
+// cache: 131,072 CRT decryptions of 2048 bits with one 32-limb lane per chain
+// took 170.5, 168.8 and 191 ms at 4, 8 and 16 steps, 19,456 of 3072 bits (48
+// limbs) 85.0, 81.9 and 80.5 ms, 65,536 of 2048 bits with 16 limbs a lane 97.4,
+// 91.0 and 87.7 ms.
+template <int TC, int L>
+constexpr int kSqUnroll = TC == 1 && L == 32 ? 8 : 16;
+
 // z = (x * y [+ x2 * y2]) / rho in both chains, chain 0's m entering chain 1.
 // y: this lane's multiplier limbs in shared memory (limb 0), doubled when
 // `dbl` is 1.  kTwo adds the second product row.  z may alias x.
@@ -139,43 +149,24 @@ template <int TC, int L, bool kTwo, class Mod>
 __device__ __forceinline__ void sq_pass(uint32_t (&z)[L], const uint32_t (&x)[L], const uint32_t* y, uint32_t dbl,
                                         const uint32_t (&x2)[L], const uint32_t* y2, const Mod& n, uint32_t np,
                                         const SqLanes<TC, L>& g) {
-  constexpr int H = TC * L, IPW = SqLanes<TC, L>::IPW, kU = 4;
+  constexpr int H = TC * L, IPW = SqLanes<TC, L>::IPW, kU = kSqUnroll<TC, L>;
   static_assert(H % kU == 0 && kU % 2 == 0, "unrolling");
   uint32_t E[L], O[L];
 #pragma unroll
   for (int j = 0; j < L; ++j) E[j] = O[j] = 0u;
   uint32_t ov = 0u, c1 = 0u, prev = 0u;
-  uint32_t cur[kU], cur2[kU];
-#pragma unroll
-  for (int k = 0; k < kU; ++k) {
-    cur[k] = y[k * IPW];
-    cur2[k] = kTwo ? y2[k * IPW] : 0u;
-  }
 #pragma unroll 1
   for (int i = 0; i < H; i += kU) {
-    // the next limbs' loads run under this round's rows (the last round's
-    // re-read the first limbs)
-    uint32_t nxt[kU], nxt2[kU];
-    const int at = i + kU < H ? i + kU : 0;
-#pragma unroll
-    for (int k = 0; k < kU; ++k) {
-      nxt[k] = y[(at + k) * IPW];
-      nxt2[k] = kTwo ? y2[(at + k) * IPW] : 0u;
-    }
 #pragma unroll
     for (int k = 0; k < kU; k += 2) {
-      row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, cur[k], dbl));
-      if constexpr (kTwo) row_mac<L>(E, O, ov, 0u, x2, g.c ? cur2[k] : 0u);
+      const uint32_t ya = y[(i + k) * IPW], yb = y[(i + k + 1) * IPW];
+      row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, ya, dbl));
+      if constexpr (kTwo) row_mac<L>(E, O, ov, 0u, x2, g.c ? y2[(i + k) * IPW] : 0u);
       sq_reduce_step<TC, L>(E, O, ov, c1, n, np, 0u, g);
-      row_mac<L>(O, E, ov, c1, x, __funnelshift_l(cur[k], cur[k + 1], dbl));
-      if constexpr (kTwo) row_mac<L>(O, E, ov, 0u, x2, g.c ? cur2[k + 1] : 0u);
+      row_mac<L>(O, E, ov, c1, x, __funnelshift_l(ya, yb, dbl));
+      if constexpr (kTwo) row_mac<L>(O, E, ov, 0u, x2, g.c ? y2[(i + k + 1) * IPW] : 0u);
       sq_reduce_step<TC, L>(O, E, ov, c1, n, np, 0u, g);
-      prev = cur[k + 1];
-    }
-#pragma unroll
-    for (int k = 0; k < kU; ++k) {
-      cur[k] = nxt[k];
-      cur2[k] = nxt2[k];
+      prev = yb;
     }
   }
   // the extra limb of rho: a doubled multiplier's top bit, or no product

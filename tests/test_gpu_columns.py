@@ -2,9 +2,11 @@
 all-zero limbs, 0, 1 and the modulus less one, for ordinary keys and for keys
 whose primes (and so n and n^2) have nothing but ones in their top limbs."""
 
+import numpy as np
 import pytest
 
 import heu_gb300 as hg
+from heu_gb300 import autotune
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +60,54 @@ def test_products_at_carry_edges(edge_key, bits, dense):
     for x in c[1:]:
         prod = prod * x * rinv % n2
     assert hg.limbs_to_ints(key.sum(hg.ints_to_limbs(c, S))) == [prod]
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("bits", [1024, 2048, 3072])
+def test_decrypt_in_every_layout(edge_key, bits, dense):
+    """Lengths on both sides of the points where the decryption takes another
+    layout (lanes per chain), ragged against the ciphertexts of a warp."""
+    key, n, _, _, _ = edge_key(bits, dense)
+    rng = np.random.default_rng(bits + dense)
+    count = 11001 if bits < 3072 else 5003
+    m = rng.integers(-(2 ** 63), 2 ** 63 - 1, count)
+    m[:4] = [0, -1, 2 ** 63 - 1, -(2 ** 63)]
+    r = rng.integers(0, 2 ** 32, (count, key.r_limbs), dtype=np.uint32)
+    ct = key.encrypt(m, r)
+    cfg = autotune.get_config(key)
+    for variant in (0, 1):
+        autotune.set_config(key, dict(cfg, dec_variant=variant))
+        for length in (1, 2, 15, 17, 33, 500, 1000, 1601, 3001, count):
+            got, ovf = key.decrypt(ct[:length])
+            assert np.array_equal(got, m[:length]) and not ovf.any(), (variant, length)
+    for window in (2, 7):
+        autotune.set_config(key, dict(cfg, dec_window=window))
+        assert np.array_equal(key.decrypt(ct[:33])[0], m[:33]), window
+    autotune.set_config(key, cfg)
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("bits", [1024, 2048, 3072])
+def test_decrypt_full_range_and_non_units(edge_key, bits, dense):
+    """Plaintexts up to +-n/2, and numbers that share a prime with n (never a
+    ciphertext): L(0) is taken as (2^(32 H) - 1) / p mod 2^(32 H)."""
+    key, n, h_s, p, q = edge_key(bits, dense)
+    n2, S, H = n * n, key.ct_limbs, key.ct_limbs // 4
+    R = 2 ** (32 * S)
+    ms = [n // 2, -(n // 2), n // 2 - 1, 1 - n // 2, 2 ** (bits // 2), 1, 0, -1]
+    zs = [pow(h_s, 12345 + i, n2) * (1 + m * n) % n2 for i, m in enumerate(ms)]
+    assert key.decrypt_bn(hg.ints_to_limbs([z * R % n2 for z in zs], S)) == ms
+
+    def side(c, pr):
+        y = pow(c, pr - 1, pr * pr)
+        hv = pow((pow(n + 1, pr - 1, pr * pr) - 1) // pr, -1, pr)
+        lv = ((y - 1) % 2 ** (32 * H)) * pow(pr, -1, 2 ** (32 * H)) % 2 ** (32 * H)
+        return lv * hv % pr
+
+    odd = [0, p, q, p * p, 5 * q * q, p * q, 7 * p]
+    want = []
+    for c in odd:
+        mp, mq = side(c, p), side(c, q)
+        m = mp + p * ((mq - mp) * pow(p, -1, q) % q)
+        want.append(m - n if m > n // 2 else m)
+    assert key.decrypt_bn(hg.ints_to_limbs([c * R % n2 for c in odd], S)) == want
