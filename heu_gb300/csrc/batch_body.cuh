@@ -18,13 +18,17 @@
 
 #include "batch.cuh"
 #include "paillier_ops.cuh"
+#include "sq_encrypt.cuh"
 
 namespace hg {
 
 namespace batch_detail {
 constexpr int kBlock = 128;
 constexpr int kWarps = kBlock / 32;
-constexpr int kYsmWordsPerWarp = 32 * 24;  // 32 * max LP over every variant
+// Shared words of a warp: 32 limbs a lane of the decryption's hand-off (up to
+// 24 limbs a lane), 5 x 16 of the encryption's areas (up to 16, 32 and 6).
+template <int V>
+constexpr int kAreaWords = V == 1 ? 80 * 32 : V == 0 ? 80 * 16 : 768;
 }  // namespace batch_detail
 
 template <int V, int S>
@@ -55,7 +59,20 @@ __device__ __forceinline__ void run_tile(const BatchJob& job, const BatchTile& t
   load_slice<L>(N, job.kc.N + g.t * L);
   const int lane_inst = lane / TPI;
   constexpr int IPW = 32 / TPI;
-  if (job.op == kBatchEncrypt) {
+  if (job.op == kBatchEncrypt && job.kc.two_digit) {
+    const SqLanes<TPI / 2, L> sg;
+    uint32_t n[L];
+    load_slice<L>(n, job.kc.n + sg.t * L);
+    const EncArgs a{EncMode::kEncrypt, (const int64_t*)job.in0, nullptr, nullptr, (const uint32_t*)job.in1, nullptr,
+                    Codec{}};
+    for (size_t wbase = tile.start; wbase < end; wbase += IPW) {
+      const size_t inst = wbase + lane_inst;
+      const bool active = inst < end;
+      __syncwarp();
+      sq_encrypt<TPI / 2, L, 1>(n, job.kc, a, (uint32_t*)job.out, active ? inst : end - 1, active, ysm, nullptr, err,
+                                sg);
+    }
+  } else if (job.op == kBatchEncrypt) {
     for (size_t wbase = tile.start; wbase < end; wbase += IPW) {
       const size_t inst = wbase + lane_inst;
       const bool active = inst < end;
@@ -87,7 +104,7 @@ __global__ void __launch_bounds__(batch_detail::kBlock) k_batch(const BatchJob* 
                                                   const BatchTile* __restrict__ tiles, uint32_t ntiles,
                                                   uint32_t* __restrict__ counter, uint32_t* __restrict__ scratch,
                                                   size_t warp_words, uint32_t* err) {
-  __shared__ __align__(16) uint32_t ysm[batch_detail::kWarps][batch_detail::kYsmWordsPerWarp];
+  __shared__ __align__(16) uint32_t ysm[batch_detail::kWarps][batch_detail::kAreaWords<V>];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   uint32_t* ws = scratch + ((size_t)blockIdx.x * batch_detail::kWarps + wib) * warp_words;
   while (true) {

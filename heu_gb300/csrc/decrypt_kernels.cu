@@ -9,7 +9,7 @@
 // 8 H^2 of a Montgomery product modulo p^2, and a chain of a prime's limbs in
 // one lane needs no shuffles but one and reads the prime from the constant
 // bank.  65,536 decryptions on GB300: 206 ms with 64-bit rows modulo p^2, 160 ms
-// with the columns of mont.cuh, 89 ms in two digits (84% of the issue bound of
+// with the columns of mont.cuh, 87 ms in two digits (84% of the issue bound of
 // the products it makes).
 #include <algorithm>
 #include <atomic>
@@ -72,26 +72,6 @@ __device__ __forceinline__ void table_store(uint32_t* tb, int e, uint32_t lane, 
   }
 }
 
-// c < n^2 (decryptor.cc:21-23), over all lanes of the instance.
-template <int TC, int L>
-__device__ __forceinline__ bool raw_below(const uint32_t* __restrict__ c, const uint32_t* __restrict__ N) {
-  constexpr int W = 2 * L;  // limbs per lane: 2 TC lanes hold 4 H
-  const Group<2 * TC> g;
-  const uint32_t* a = c + g.t * W;
-  const uint32_t* b = N + g.t * W;
-  uint32_t borrow = 0u;
-  bool same = true;
-#pragma unroll 4
-  for (int j = 0; j < W; ++j) {
-    const uint64_t d = (uint64_t)a[j] - b[j] - borrow;
-    borrow = (uint32_t)(d >> 63);
-    same = same && a[j] == b[j];
-  }
-  uint32_t out;
-  (void)lookahead<2 * TC>(g, borrow != 0u, same, 0u, out);
-  return out != 0u;
-}
-
 // One side of a warp's instances: digit 1 of c^(p-1) mod p^2, to
 // z[(2 i + side) H ..].  The exponent program and its table (2^(wd-1) odd
 // powers, then the square) are as in build_prog.
@@ -106,7 +86,8 @@ __device__ __forceinline__ void dec_pow_side(const Mod& n, const KeyConst& kc, c
   const int ntab = 1 << (sc.wd - 1);
   const uint32_t* src = ct + i * (4 * H);
   if (side == 0) {
-    const bool ok = raw_below<TC, L>(src, kc.N);
+    // c < n^2 (decryptor.cc:21-23)
+    const bool ok = raw_below<TC, 2 * L>(src, kc.N);
     if (active && !ok && g.lane == g.base) atomicOr(err, kErrCtRange);
   }
   uint32_t x[L];
@@ -130,12 +111,12 @@ __device__ __forceinline__ void dec_pow_side(const Mod& n, const KeyConst& kc, c
     if (s == ntab) table_load<L>(x, tb, sc.start[side], g.lane);
     sq_stage<TC, L>(area, x, e >= 0, g);
     if (e < 0) {
-      sq_pass<TC, L, false>(x, x, g.limb(area, 0, 0), (uint32_t)g.c, x, nullptr, n, np, g);
+      sq_pass<TC, L, false>(x, x, g.limb(area, 0, 0), (uint32_t)g.c, 0u, x, nullptr, n, np, g);
     } else {
       uint32_t y0[L];
       table_load<L>(x, tb, e, g.lane);
       table_load<L>(y0, tb, e, g.lane - g.c * TC);
-      sq_pass<TC, L, true>(x, x, g.limb(area, 0, 0), 0u, y0, g.limb(area, 1, 0), n, np, g);
+      sq_pass<TC, L, true>(x, x, g.limb(area, 0, 0), 0u, 0u, y0, g.limb(area, 1, 0), n, np, g);
     }
     if (s < ntab) table_store<L>(tb, s == 0 ? ntab : s, g.lane, x);
   }
@@ -165,7 +146,7 @@ __global__ void __launch_bounds__(32, dec_min_blocks(L))
               const __grid_constant__ SecConst sc, const uint32_t* __restrict__ ct, size_t count,
               uint32_t* __restrict__ scratch, uint32_t* __restrict__ z, uint32_t* err, unsigned long long* ctr) {
   using G = SqLanes<TC, L>;
-  __shared__ uint32_t area[G::kWords];
+  __shared__ __align__(16) uint32_t area[2 * G::kDigit];
   const G g;
   const size_t slots = ((size_t)1 << (sc.wd - 1)) + 1;
   uint32_t* tb = scratch + (size_t)blockIdx.x * slots * 32 * L;

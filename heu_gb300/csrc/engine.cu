@@ -175,6 +175,8 @@ struct KeyRec {
   bool secret = false;
   BN n, N, hs, p, q;
   DevBuf consts, sconsts, table, progs;
+  DevBuf sqconsts;            // two-digit encryption: e0 e1 rz (S each), rho2, nrho2 (H each)
+  std::vector<uint32_t> hn;   // n (S/2 limbs)
   hg::KeyConst kc{};
   hg::SecConst sc{};
   int grid_mul = 0;
@@ -451,14 +453,24 @@ void ou_plain_pow(KeyRec& k, Work& w, const int64_t* m, int negate, const uint32
                "OU H pass");
 }
 
+// ZPaillier encryption: in two digits, or modulo n^2 for a key whose h_s is no
+// unit.
+void encrypt_zp(KeyRec& k, Work& w, const hg::EncArgs& a, uint32_t* out, size_t count) {
+  if (k.kc.two_digit)
+    cuda_check(hg::launch_sq_encrypt(k.S, k.kc, a, out, count, w.errp(), w.stream), "encrypt launch");
+  else
+    cuda_check(hg::launch_encrypt(k.S, k.kc, a.mode, a.m, a.m_mag, a.m_neg, a.r, a.ct_in, out, count, w.errp(), 0,
+                                  w.stream, a.cd),
+               "encrypt launch");
+}
+
 void core_encrypt(KeyRec& k, Work& w, hg::EncMode mode, const int64_t* m, const uint32_t* m_mag,
                   const uint8_t* m_neg, const uint32_t* r, const uint32_t* ct_in, uint32_t* out, size_t count) {
   if (k.scheme == 1 && mode == hg::EncMode::kEncrypt) {
     ou_plain_pow(k, w, m, 0, m_mag, m_neg, r, nullptr, out, count);
     return;
   }
-  cuda_check(hg::launch_encrypt(k.S, k.kc, mode, m, m_mag, m_neg, r, ct_in, out, count, w.errp(), 0, w.stream),
-             "encrypt launch");
+  encrypt_zp(k, w, hg::EncArgs{mode, m, m_mag, m_neg, r, ct_in, hg::Codec{}}, out, count);
 }
 
 // Device encodings (PlainEncoder / BatchEncoder) of the C-ABI's HG_CODEC_*.
@@ -480,9 +492,9 @@ hg::Codec make_codec(const KeyRec& k, int codec, int64_t scale, int padding, con
 
 void core_encrypt_encoded(KeyRec& k, Work& w, const void* values, const uint32_t* r, uint32_t* out, size_t count,
                           const hg::Codec& cd) {
-  cuda_check(hg::launch_encrypt(k.S, k.kc, hg::EncMode::kEncrypt, static_cast<const int64_t*>(values), nullptr,
-                                nullptr, r, nullptr, out, count, w.errp(), 0, w.stream, cd),
-             "encrypt launch");
+  encrypt_zp(k, w,
+             hg::EncArgs{hg::EncMode::kEncrypt, static_cast<const int64_t*>(values), nullptr, nullptr, r, nullptr, cd},
+             out, count);
 }
 
 // CRT decryption into any of the output forms.
@@ -850,6 +862,93 @@ void core_matmul_bn(KeyRec& k, Work& w, const uint32_t* x, size_t M, size_t K, c
                      [&](size_t kk, size_t j, int plane) { return ys[kk * N + j].bit((size_t)plane); }, o, out);
 }
 
+// Fixed-base table of `base_mont` powers over the modulus of `t` (npos x
+// (2^w - 1) entries, Montgomery form), the layout k_encrypt reads.
+void build_fixed_base(int S, hg::KeyConst& t, DevBuf& buf, const uint32_t* base_mont, int exp_bits, int window) {
+  t.w = window;
+  t.rbits = exp_bits;
+  t.npos = (exp_bits + window - 1) / window;
+  const size_t ent = ((size_t)1 << window) - 1;
+  t.table = buf.ensure<uint32_t>((size_t)t.npos * ent * S * 4);
+  DevBuf bases;
+  uint32_t* b = bases.ensure<uint32_t>((size_t)t.npos * S * 4);
+  cuda_check(hg::launch_table_bases(S, t, base_mont, b, nullptr), "table bases");
+  cuda_check(hg::launch_table_level(S, t, const_cast<uint32_t*>(t.table), b, -1, nullptr), "table level");
+  for (int lv = 0; lv < window; ++lv)
+    cuda_check(hg::launch_table_level(S, t, const_cast<uint32_t*>(t.table), b, lv, nullptr), "table level");
+  cuda_check(cudaDeviceSynchronize(), "table build");
+}
+
+// Table and constants of the two-digit encryption (sq_encrypt.cuh); false
+// where h_s is not a unit modulo n.
+bool build_sq_table(KeyRec& k) {
+  hg::KeyConst& kc = k.kc;
+  const int S = k.S;
+  const size_t H = (size_t)S / 2;
+  const BN &n = k.n, &N = k.N;
+  const BN rho = BN(1).shl(32 * (H + 1));
+  const BN rho1 = rho % n, rho2 = (rho1 * rho1) % n;
+  // digits of v modulo n^2: v = x0 - x1 n
+  auto digit1 = [&](const BN& v) {
+    const BN t = (v / n) % n;
+    return t.is_zero() ? t : n - t;
+  };
+  const BN h = (k.hs * (rho % N)) % N;  // h_s rho
+  const BN h0 = h % n;
+  BN ih;
+  try {
+    ih = (BN::invmod(h0, n) * rho2) % n;
+  } catch (const std::runtime_error&) {
+    return false;
+  }
+  const BN ir = BN::invmod(rho1, n);  // rho^-1
+  // entry (v0 | v1 / v0 rho) of v, given v0^-1 mod n
+  std::vector<uint32_t> hc(3 * (size_t)S + 6 * H);
+  auto entry = [&](size_t at, const BN& v, const BN& inv0) {
+    (v % n).to_limbs(hc.data() + at, H);
+    ((((digit1(v) * inv0) % n) * rho1) % n).to_limbs(hc.data() + at + H, H);
+  };
+  // 2^(32 S) rho = rho^3 / 2^64;  rho;  rho^3 / 2^(32 S) = 2^(32 H + 96)
+  entry(0, BN(1).shl(96 * H + 32) % N, (((ir * ir) % n) * ((ir * BN(1).shl(64)) % n)) % n);
+  entry(S, rho % N, ir);
+  entry(2 * (size_t)S, BN(1).shl(32 * H + 96) % N, (((ir * ir) % n) * (BN(1).shl(32 * H - 32) % n)) % n);
+  rho2.to_limbs(hc.data() + 3 * (size_t)S, H);
+  (n - rho2).to_limbs(hc.data() + 3 * (size_t)S + H, H);
+  const size_t first = 3 * (size_t)S + 2 * H;
+  h0.to_limbs(hc.data() + first, H);
+  digit1(h).to_limbs(hc.data() + first + H, H);
+  ih.to_limbs(hc.data() + first + 2 * H, H);
+  ((ir * BN(1).shl(64)) % n).to_limbs(hc.data() + first + 3 * H, H);  // rho^2 / (2^(32 S) rho)
+  uint32_t* d = k.sqconsts.ensure<uint32_t>(hc.size() * 4);
+  cuda_check(cudaMemcpy(d, hc.data(), hc.size() * 4, cudaMemcpyHostToDevice), "upload consts");
+  k.hn.assign(H, 0u);
+  n.to_limbs(k.hn.data(), H);
+  kc.npn = neg_inv32(n.d[0]);
+  kc.e0 = d;
+  kc.ie0 = d + first + 3 * H;
+  kc.e1 = d + S;
+  kc.rz = d + 2 * S;
+  kc.rho2 = d + 3 * S;
+  kc.nrho2 = d + 3 * S + H;
+  kc.hn = k.hn.data();
+  const size_t ent = ((size_t)1 << kc.w) - 1;
+  uint32_t* tab = k.table.ensure<uint32_t>((size_t)kc.npos * ent * S * 4);
+  kc.table = tab;
+  // the inverses of a few positions at a time: at most 1 GiB beside the table
+  const int step = (int)std::max<size_t>(1, std::min<size_t>((size_t)kc.npos, ((size_t)1 << 30) / (ent * H * 4)));
+  DevBuf bases, inv;
+  uint32_t* b = bases.ensure<uint32_t>((size_t)kc.npos * 3 * H * 4);
+  uint32_t* iv = inv.ensure<uint32_t>((size_t)step * ent * H * 4);
+  cuda_check(hg::launch_sq_bases(S, kc, d + first, b, nullptr), "table bases");
+  for (int p0 = 0; p0 < kc.npos; p0 += step)
+    for (int lv = -1; lv < kc.w + (p0 == 0 ? 1 : 0); ++lv)
+      cuda_check(hg::launch_sq_level(S, kc, tab, iv, b, p0, lv < kc.w ? std::min(step, kc.npos - p0) : 1, lv, nullptr),
+                 "table level");
+  cuda_check(cudaDeviceSynchronize(), "table build");
+  kc.two_digit = 1;
+  return true;
+}
+
 int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t* hs_l, const uint32_t* p_l,
                  const uint32_t* q_l, int window) {
   if (key_bits % 64 != 0) fail(HG_ERR_UNSUPPORTED, "key size must be a multiple of 64 bits");
@@ -900,17 +999,7 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
   kc.rlimbs = (int)key_bits / 64;
   kc.npos = (kc.rbits + kc.w - 1) / kc.w;
   // fixed-base table on the device
-  const size_t ent = ((size_t)1 << kc.w) - 1;
-  uint32_t* tab = k->table.ensure<uint32_t>((size_t)kc.npos * ent * S * 4);
-  kc.table = tab;
-  {
-    DevBuf bases;
-    uint32_t* b = bases.ensure<uint32_t>((size_t)kc.npos * S * 4);
-    cuda_check(hg::launch_table_bases(S, kc, dc + 5 * S, b, nullptr), "table bases");
-    cuda_check(hg::launch_table_level(S, kc, tab, b, -1, nullptr), "table level");
-    for (int lv = 0; lv < kc.w; ++lv) cuda_check(hg::launch_table_level(S, kc, tab, b, lv, nullptr), "table level");
-    cuda_check(cudaDeviceSynchronize(), "table build");
-  }
+  if (!build_sq_table(*k)) build_fixed_base(S, kc, k->table, dc + 5 * S, kc.rbits, kc.w);
   kc.variant = 0;
   k->grid_mul = hg::resident_blocks_mul(S, 0);
   if (p_l && q_l) {
@@ -999,23 +1088,6 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
   const int id = ctx->next_key++;
   ctx->keys[id] = std::move(k);
   return id;
-}
-
-// Fixed-base table of `base_mont` powers over the modulus of `t` (npos x
-// (2^w - 1) entries, Montgomery form), the layout k_encrypt reads.
-void build_fixed_base(int S, hg::KeyConst& t, DevBuf& buf, const uint32_t* base_mont, int exp_bits, int window) {
-  t.w = window;
-  t.rbits = exp_bits;
-  t.npos = (exp_bits + window - 1) / window;
-  const size_t ent = ((size_t)1 << window) - 1;
-  t.table = buf.ensure<uint32_t>((size_t)t.npos * ent * S * 4);
-  DevBuf bases;
-  uint32_t* b = bases.ensure<uint32_t>((size_t)t.npos * S * 4);
-  cuda_check(hg::launch_table_bases(S, t, base_mont, b, nullptr), "table bases");
-  cuda_check(hg::launch_table_level(S, t, const_cast<uint32_t*>(t.table), b, -1, nullptr), "table level");
-  for (int lv = 0; lv < window; ++lv)
-    cuda_check(hg::launch_table_level(S, t, const_cast<uint32_t*>(t.table), b, lv, nullptr), "table level");
-  cuda_check(cudaDeviceSynchronize(), "table build");
 }
 
 int ou_random_bits(size_t n_bits) {  // ou/encryptor.cc:12-20, public_key.h:27-31

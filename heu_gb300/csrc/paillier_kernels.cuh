@@ -33,6 +33,18 @@ struct KeyConst {
   int rbits;            // bits of the encryption randomness r (k/2)
   int rlimbs;           // 32-bit limbs per r
   int variant;          // (threads per instance, limbs per thread) variant, 0 or 1
+  // two-digit encryption (sq_encrypt.cuh; H = S/2 limbs of n, rho = 2^(32 (H+1))):
+  // the table then holds entries (Y0 | y), Montgomery form of radix rho, those
+  // of position 0 times 2^(32 S), the radix of the output
+  int two_digit;          // 0: N is no square, or h_s shares a factor with it
+  uint32_t npn;           // -n^-1 mod 2^32
+  const uint32_t* e0;     // entry of 2^(32 S), for a zero digit at position 0  (S limbs)
+  const uint32_t* ie0;    // rho^2 / Y0 mod n of e0                            (H limbs)
+  const uint32_t* e1;     // entry of 1, for a zero digit elsewhere            (S limbs)
+  const uint32_t* rz;     // entry of rho^2 / 2^(32 S), for randomizing        (S limbs)
+  const uint32_t* rho2;   // rho^2 mod n   (H limbs)
+  const uint32_t* nrho2;  // -rho^2 mod n  (H limbs)
+  const uint32_t* hn;     // n on the host (H limbs)
 };
 
 // Secret-key constants for CRT decryption.  Index 0 = p side, 1 = q side.
@@ -94,6 +106,17 @@ struct Codec {
   void* out1;       // decryption: the second slot's values (batch kinds)
 };
 
+// What one encryption reads; `m` holds the values to encode with a codec.
+struct EncArgs {
+  EncMode mode;
+  const int64_t* m;
+  const uint32_t* m_mag;
+  const uint8_t* m_neg;
+  const uint32_t* r;
+  const uint32_t* ct_in;
+  Codec cd;
+};
+
 // Launchers.  All are asynchronous on `stream` and return cudaError_t of the
 // launch.  `cfg` selects the (threads per instance, limbs per thread) variant.
 // With cd.kind != kCodecNone (mode kEncrypt) `m` holds the values to encode
@@ -101,6 +124,16 @@ struct Codec {
 cudaError_t launch_encrypt(int S, const KeyConst& kc, EncMode mode, const int64_t* m, const uint32_t* m_mag,
                            const uint8_t* m_neg, const uint32_t* r, const uint32_t* ct_in, uint32_t* out,
                            size_t count, uint32_t* err, int grid, cudaStream_t st, const Codec& cd = Codec{});
+// The same for two-digit keys (encrypt_kernels.cu).
+cudaError_t launch_sq_encrypt(int S, const KeyConst& kc, const EncArgs& a, uint32_t* out, size_t count, uint32_t* err,
+                              cudaStream_t st);
+// Their tables: bases (3 H limbs a position) from the digits of h_s rho and
+// rho^2 / X0 mod n (`first`, 3 H limbs), then the levels -1, 0 .. w - 1 of the
+// entries of npos positions from pos0, whose inverses are in `inv` (H limbs an
+// entry of those positions); level w multiplies position 0 by 2^(32 S).
+cudaError_t launch_sq_bases(int S, const KeyConst& kc, const uint32_t* first, uint32_t* bases, cudaStream_t st);
+cudaError_t launch_sq_level(int S, const KeyConst& kc, uint32_t* table, uint32_t* inv, const uint32_t* bases, int pos0,
+                            int npos, int level, cudaStream_t st);
 cudaError_t launch_add(int S, const KeyConst& kc, const uint32_t* a, const uint32_t* b, uint32_t* out,
                        size_t count, uint32_t* err, cudaStream_t st);
 cudaError_t launch_add_plain(int S, const KeyConst& kc, const uint32_t* a, const int64_t* p, int neg_p,

@@ -20,9 +20,10 @@
 // subtraction is needed unless n's top limb is all ones; that case is handled
 // behind one vote per pass.
 //
-// Multiplier limbs come from shared memory, [digit][limb][instance of the
-// warp], multiplicands and running columns (mont.cuh) from registers.  n is
-// any array of L words: registers, or with TC = 1 the kernel's constant bank,
+// Multiplier limbs come from shared memory in quads, [digit][limb / 4]
+// [instance of the warp][4], so one 16-byte load feeds four steps;
+// multiplicands and running columns (mont.cuh) are in registers.  n is any
+// array of L words: registers, or with TC = 1 the kernel's constant bank,
 // which frees L registers.
 #pragma once
 #include "mont.cuh"
@@ -33,9 +34,9 @@ template <int TC, int L>
 struct SqLanes {
   static constexpr int H = TC * L;
   static constexpr int IPW = 32 / (2 * TC);      // instances per warp
-  static constexpr int kDigit = H * IPW + (IPW == 16 ? 16 : 0);  // words between the digits' areas
-  static constexpr int kWords = 2 * kDigit;      // shared words per warp
-  uint32_t lane, base, chain_base;  // warp lane; first lane of the group and of the chain
+  static constexpr int kDigit = H * IPW;         // shared words per digit and warp
+  static constexpr int kVec = L % 4 == 0 ? 4 : 2;  // words of a lane's vector accesses
+  uint32_t lane, base;  // warp lane; the group's first lane
   int c, t, iw;                     // chain, lane in the chain, instance of the warp
   __device__ __forceinline__ SqLanes() {
     lane = threadIdx.x & 31u;
@@ -43,29 +44,65 @@ struct SqLanes {
     c = (int)(lane / TC) & 1;
     t = (int)(lane % TC);
     base = (uint32_t)iw * 2 * TC;
-    chain_base = base + (uint32_t)c * TC;
   }
-  // this lane's slice of digit d in the warp's area
+  // limb i (a multiple of 4) of digit d of this lane's instance
   __device__ __forceinline__ uint32_t* limb(uint32_t* area, int d, int i) const {
-    return area + d * kDigit + i * IPW + iw;
+    return area + d * kDigit + (i * IPW + iw * 4);
+  }
+  // word offset, from limb 0, of vector v of this lane's slice
+  __device__ __forceinline__ int slice_at(int v) const {
+    const int i = t * L + v * kVec;
+    return (i >> 2) * 4 * IPW + (i & 3);
   }
 };
+
+// This lane's slice to and from a digit's area (`digit` points at its limb 0
+// of the instance).
+template <int TC, int L>
+__device__ __forceinline__ void sq_put(uint32_t* digit, const uint32_t (&x)[L], const SqLanes<TC, L>& g) {
+  constexpr int V = SqLanes<TC, L>::kVec;
+#pragma unroll
+  for (int v = 0; v < L / V; ++v) {
+    uint32_t* p = digit + g.slice_at(v);
+    if constexpr (V == 4)
+      *reinterpret_cast<uint4*>(p) = make_uint4(x[4 * v], x[4 * v + 1], x[4 * v + 2], x[4 * v + 3]);
+    else
+      *reinterpret_cast<uint2*>(p) = make_uint2(x[2 * v], x[2 * v + 1]);
+  }
+}
+
+template <int TC, int L>
+__device__ __forceinline__ void sq_get(uint32_t (&x)[L], const uint32_t* digit, const SqLanes<TC, L>& g) {
+  constexpr int V = SqLanes<TC, L>::kVec;
+#pragma unroll
+  for (int v = 0; v < L / V; ++v) {
+    const uint32_t* p = digit + g.slice_at(v);
+    if constexpr (V == 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(p);
+      x[4 * v] = q.x;
+      x[4 * v + 1] = q.y;
+      x[4 * v + 2] = q.z;
+      x[4 * v + 3] = q.w;
+    } else {
+      const uint2 q = *reinterpret_cast<const uint2*>(p);
+      x[2 * v] = q.x;
+      x[2 * v + 1] = q.y;
+    }
+  }
+}
 
 // Write this lane's slice of its digit (digit 0 only if `both` is false).
 template <int TC, int L>
 __device__ __forceinline__ void sq_stage(uint32_t* area, const uint32_t (&x)[L], bool both, const SqLanes<TC, L>& g) {
   __syncwarp();
-  if (both || g.c == 0) {
-    uint32_t* s = g.limb(area, g.c, g.t * L);
-#pragma unroll
-    for (int j = 0; j < L; ++j) s[j * SqLanes<TC, L>::IPW] = x[j];
-  }
+  if (both || g.c == 0) sq_put<TC, L>(g.limb(area, g.c, 0), x, g);
   __syncwarp();
 }
 
 // Reduction of one limb in both chains, then the shift by one limb.  The
-// pending c1 must be 0.  `in` enters the top limb of chain 0.
-template <int TC, int L, class Mod>
+// pending c1 must be 0.  `in` enters the top limb of chain 0.  Without kJoin
+// the chains are two reductions modulo n of their own.
+template <int TC, int L, bool kJoin = true, class Mod>
 __device__ __forceinline__ void sq_reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t& ov, uint32_t& c1,
                                                const Mod& n, uint32_t np, uint32_t in, const SqLanes<TC, L>& g) {
   // both chains' lowest limbs travel together, so that chain 1 finds its m
@@ -73,9 +110,8 @@ __device__ __forceinline__ void sq_reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)
   const uint32_t a = __shfl_sync(kFull, Ev[0], g.base);
   const uint32_t b = TC > 1 ? __shfl_sync(kFull, Ev[0], g.base + TC) : Ev[0];
   const uint32_t m0 = a * np;
-  const uint32_t m = g.c ? (b + m0) * np : m0;
-  const uint32_t inject = (g.c == 1 && g.t == 0) ? m0 : 0u;
-  row_mac<L>(Ev, Od, ov, inject, n, m);
+  const uint32_t m = g.c ? (kJoin ? b + m0 : b) * np : m0;
+  row_mac<L>(Ev, Od, ov, (kJoin && g.c == 1 && g.t == 0) ? m0 : 0u, n, m);
   uint32_t w = 0u;
   if constexpr (TC > 1) w = __shfl_down_sync(kFull, Ev[0], 1, TC);
   if (g.t == TC - 1) w = in;
@@ -88,7 +124,7 @@ __device__ __forceinline__ void sq_reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)
 }
 
 // Columns -> limbs of both chains' results, below 2^(32 H).
-template <int TC, int L, class Mod>
+template <int TC, int L, bool kJoin = true, class Mod>
 __device__ __forceinline__ void sq_settle(uint32_t (&x)[L], const uint32_t (&Ev)[L], const uint32_t (&Od)[L],
                                           uint32_t c1, const Mod& n, const SqLanes<TC, L>& g) {
   uint32_t top;
@@ -111,7 +147,7 @@ __device__ __forceinline__ void sq_settle(uint32_t (&x)[L], const uint32_t (&Ev)
       d[j] = top ? n[j] : 0u;
       small[j] = 0u;
     }
-    if (g.c == 1 && g.t == 0 && owed) small[0] = 1u;
+    if (kJoin && g.c == 1 && g.t == 0 && owed) small[0] = 1u;
     if constexpr (TC == 1) {
       x[0] = sub_cc(x[0], d[0]);
 #pragma unroll
@@ -135,7 +171,7 @@ __device__ __forceinline__ void sq_settle(uint32_t (&x)[L], const uint32_t (&Ev)
 // cache: 131,072 CRT decryptions of 2048 bits with one 32-limb lane per chain
 // took 170.5, 168.8 and 191 ms at 4, 8 and 16 steps, 19,456 of 3072 bits (48
 // limbs) 85.0, 81.9 and 80.5 ms, 65,536 of 2048 bits with 16 limbs a lane 97.4,
-// 91.0 and 87.7 ms.
+// 91.0 and 87.7 ms.  (Multipliers in 16-byte loads then took 1 to 3% off each.)
 template <int TC, int L>
 constexpr int kSqUnroll = TC == 1 && L == 32 ? 8 : 16;
 
@@ -145,12 +181,15 @@ constexpr int kSqUnroll = TC == 1 && L == 32 ? 8 : 16;
 //   square:           x = own digit, y = digit 0, dbl = chain
 //   product with Y:   x = Y's digit of the chain, y = X0, x2 = Y0, y2 = X1 (chain 1)
 //   times integer Y0: x = Y0, y = own digit of X
-template <int TC, int L, bool kTwo, class Mod>
+// kJoin = false: z_c = x_c * y_c / rho modulo n in each chain for itself.
+// `ytop` is limb H of an undoubled multiplier (a few units: the result's
+// bound holds).
+template <int TC, int L, bool kTwo, bool kJoin = true, class Mod>
 __device__ __forceinline__ void sq_pass(uint32_t (&z)[L], const uint32_t (&x)[L], const uint32_t* y, uint32_t dbl,
-                                        const uint32_t (&x2)[L], const uint32_t* y2, const Mod& n, uint32_t np,
-                                        const SqLanes<TC, L>& g) {
+                                        uint32_t ytop, const uint32_t (&x2)[L], const uint32_t* y2, const Mod& n,
+                                        uint32_t np, const SqLanes<TC, L>& g) {
   constexpr int H = TC * L, IPW = SqLanes<TC, L>::IPW, kU = kSqUnroll<TC, L>;
-  static_assert(H % kU == 0 && kU % 2 == 0, "unrolling");
+  static_assert(H % kU == 0 && kU % 4 == 0, "unrolling");
   uint32_t E[L], O[L];
 #pragma unroll
   for (int j = 0; j < L; ++j) E[j] = O[j] = 0u;
@@ -158,21 +197,28 @@ __device__ __forceinline__ void sq_pass(uint32_t (&z)[L], const uint32_t (&x)[L]
 #pragma unroll 1
   for (int i = 0; i < H; i += kU) {
 #pragma unroll
-    for (int k = 0; k < kU; k += 2) {
-      const uint32_t ya = y[(i + k) * IPW], yb = y[(i + k + 1) * IPW];
-      row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, ya, dbl));
-      if constexpr (kTwo) row_mac<L>(E, O, ov, 0u, x2, g.c ? y2[(i + k) * IPW] : 0u);
-      sq_reduce_step<TC, L>(E, O, ov, c1, n, np, 0u, g);
-      row_mac<L>(O, E, ov, c1, x, __funnelshift_l(ya, yb, dbl));
-      if constexpr (kTwo) row_mac<L>(O, E, ov, 0u, x2, g.c ? y2[(i + k + 1) * IPW] : 0u);
-      sq_reduce_step<TC, L>(O, E, ov, c1, n, np, 0u, g);
-      prev = yb;
+    for (int k = 0; k < kU; k += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(y + (i + k) * IPW);
+      const uint4 q2 = kTwo ? *reinterpret_cast<const uint4*>(y2 + (i + k) * IPW) : make_uint4(0u, 0u, 0u, 0u);
+      row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, q.x, dbl));
+      if constexpr (kTwo) row_mac<L>(E, O, ov, 0u, x2, g.c ? q2.x : 0u);
+      sq_reduce_step<TC, L, kJoin>(E, O, ov, c1, n, np, 0u, g);
+      row_mac<L>(O, E, ov, c1, x, __funnelshift_l(q.x, q.y, dbl));
+      if constexpr (kTwo) row_mac<L>(O, E, ov, 0u, x2, g.c ? q2.y : 0u);
+      sq_reduce_step<TC, L, kJoin>(O, E, ov, c1, n, np, 0u, g);
+      row_mac<L>(E, O, ov, c1, x, __funnelshift_l(q.y, q.z, dbl));
+      if constexpr (kTwo) row_mac<L>(E, O, ov, 0u, x2, g.c ? q2.z : 0u);
+      sq_reduce_step<TC, L, kJoin>(E, O, ov, c1, n, np, 0u, g);
+      row_mac<L>(O, E, ov, c1, x, __funnelshift_l(q.z, q.w, dbl));
+      if constexpr (kTwo) row_mac<L>(O, E, ov, 0u, x2, g.c ? q2.w : 0u);
+      sq_reduce_step<TC, L, kJoin>(O, E, ov, c1, n, np, 0u, g);
+      prev = q.w;
     }
   }
-  // the extra limb of rho: a doubled multiplier's top bit, or no product
-  row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, 0u, dbl));
-  sq_reduce_step<TC, L>(E, O, ov, c1, n, np, 0u, g);
-  sq_settle<TC, L>(z, O, E, c1, n, g);
+  // the extra limb of rho: a doubled multiplier's top bit, or ytop
+  row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, ytop, dbl));
+  sq_reduce_step<TC, L, kJoin>(E, O, ov, c1, n, np, 0u, g);
+  sq_settle<TC, L, kJoin>(z, O, E, c1, n, g);
 }
 
 // One reduction step without a product row.
@@ -237,6 +283,158 @@ __device__ __forceinline__ void sq_redc(uint32_t (&z)[L], const uint32_t (&x)[L]
   }
   sq_redc_step<TC, L>(E, O, ov, c1, n, np, 0u, g);
   sq_settle<TC, L>(z, O, E, c1, n, g);
+}
+
+// ---- digit helpers over one chain -------------------------------------------
+// r = a + b over the chain's H limbs; returns the carry out (in every lane).
+template <int TC, int L>
+__device__ __forceinline__ uint32_t chain_add(uint32_t (&r)[L], const uint32_t (&a)[L], const uint32_t (&b)[L]) {
+  if constexpr (TC == 1) {
+    r[0] = add_cc(a[0], b[0]);
+#pragma unroll
+    for (int j = 1; j < L; ++j) r[j] = addc_cc(a[j], b[j]);
+    return addc(0u, 0u);
+  } else {
+    const Group<TC> cg;
+    return add_full<TC, L>(r, a, b, cg);
+  }
+}
+
+// r = a - b; returns the borrow out.
+template <int TC, int L>
+__device__ __forceinline__ uint32_t chain_sub(uint32_t (&r)[L], const uint32_t (&a)[L], const uint32_t (&b)[L]) {
+  if constexpr (TC == 1) {
+    r[0] = sub_cc(a[0], b[0]);
+#pragma unroll
+    for (int j = 1; j < L; ++j) r[j] = subc_cc(a[j], b[j]);
+    return subc(0u, 0u) & 1u;
+  } else {
+    const Group<TC> cg;
+    return sub_full<TC, L>(r, a, b, cg);
+  }
+}
+
+// x (with `top` above its limbs) less n where that is not negative.
+template <int TC, int L>
+__device__ __forceinline__ void chain_reduce_once(uint32_t (&x)[L], uint32_t top, const uint32_t (&n)[L]) {
+  uint32_t d[L];
+  const uint32_t borrow = chain_sub<TC, L>(d, x, n);
+  select_slice<L>(x, top != 0u || borrow == 0u, d, x);
+}
+
+// Limbs plus a carry word per lane -> limbs; returns the word above the top.
+template <int TC, int L>
+__device__ __forceinline__ uint32_t chain_settle(uint32_t (&x)[L], uint32_t carry) {
+  if constexpr (TC == 1) {
+    return carry;
+  } else {
+    const Group<TC> cg;
+    uint32_t c[L];
+    c[0] = __shfl_up_sync(kFull, carry, 1, TC);
+    if (cg.t == 0) c[0] = 0u;
+#pragma unroll
+    for (int j = 1; j < L; ++j) c[j] = 0u;
+    const uint32_t out = add_full<TC, L>(x, x, c, cg);
+    return __shfl_sync(kFull, carry, TC - 1, TC) + out;
+  }
+}
+
+// Is the raw number of 2 TC * W limbs at `a` below the one at `b`?
+template <int TC, int W>
+__device__ __forceinline__ bool raw_below(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b) {
+  const Group<2 * TC> g;
+  a += g.t * W;
+  b += g.t * W;
+  uint32_t borrow = 0u;
+  bool same = true;
+#pragma unroll 4
+  for (int j = 0; j < W; ++j) {
+    const uint64_t d = (uint64_t)a[j] - b[j] - borrow;
+    borrow = (uint32_t)(d >> 63);
+    same = same && a[j] == b[j];
+  }
+  uint32_t out;
+  (void)lookahead<2 * TC>(g, borrow != 0u, same, 0u, out);
+  return out != 0u;
+}
+
+// The residue x / rho as a raw number below n^2: chain c gets limbs
+// [c H + t L, c H + t L + L) of it.  `area` holds two digits.
+//   x / rho = x0 - x1 n with 0 <= x0 <= n, 0 <= x1 <= n + 1, and then
+//   x0 + (n - x1) n with both digits in [0, n).
+template <int TC, int L, class Mod>
+__device__ __forceinline__ void sq_to_raw(uint32_t (&r)[L], const uint32_t (&xin)[L], uint32_t* area, const Mod& n,
+                                          uint32_t np, const SqLanes<TC, L>& g) {
+  constexpr int H = TC * L, IPW = SqLanes<TC, L>::IPW;
+  uint32_t x[L], v[L], nn[L], d[L];
+  sq_redc<TC, L>(x, xin, n, np, g);
+#pragma unroll
+  for (int j = 0; j < L; ++j) nn[j] = n[j];
+  // both digits below n; x0 = n is 0 and owes 1 to digit 1
+  const bool whole = chain_sub<TC, L>(d, x, nn) == 0u;
+  const bool owed = __shfl_sync(kFull, (int)whole, g.base) != 0;
+  select_slice<L>(x, whole, d, x);
+  // v = n - x1 + owed mod n (chain 1)
+  (void)chain_sub<TC, L>(v, nn, x);
+#pragma unroll
+  for (int j = 0; j < L; ++j) d[j] = 0u;
+  if (g.t == 0 && owed) d[0] = 1u;
+  const uint32_t top = chain_add<TC, L>(v, v, d);
+  chain_reduce_once<TC, L>(v, top, nn);
+  __syncwarp();
+  if (g.c == 1) sq_put<TC, L>(g.limb(area, 1, 0), v, g);
+  __syncwarp();
+  // x0 + v n: rows of n, the lowest limb leaves in every step
+  const uint32_t* y = g.limb(area, 1, 0);
+  uint32_t* low = g.limb(area, 0, 0);
+  uint32_t E[L], O[L], ov = 0u, c1 = 0u;
+#pragma unroll
+  for (int j = 0; j < L; ++j) {
+    E[j] = x[j];
+    O[j] = 0u;
+  }
+  auto step = [&](uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t w) {
+    row_mac<L>(Ev, Od, ov, c1, nn, w);
+    const uint32_t out = Ev[0];
+    if constexpr (TC == 1) {
+      c1 = Ev[1];
+#pragma unroll
+      for (int j = 0; j + 2 < L; ++j) Ev[j] = Ev[j + 2];
+      Ev[L - 2] = 0u;
+      Ev[L - 1] = ov;
+      ov = 0u;
+    } else {
+      const Group<TC> cg;
+      shift_limb<TC, L>(Ev, ov, c1, cg);
+    }
+    return out;
+  };
+#pragma unroll 1
+  for (int i = 0; i < H; i += 4) {
+    const uint4 q = *reinterpret_cast<const uint4*>(y + i * IPW);
+    uint4 o;
+    o.x = step(E, O, q.x);
+    o.y = step(O, E, q.y);
+    o.z = step(E, O, q.z);
+    o.w = step(O, E, q.w);
+    if (g.c == 0 && g.t == 0) *reinterpret_cast<uint4*>(low + i * IPW) = o;
+  }
+  if constexpr (TC == 1) {
+    x[0] = add_cc(E[0], c1);
+#pragma unroll
+    for (int j = 1; j < L; ++j) x[j] = addc_cc(E[j], O[j - 1]);
+    (void)addc(0u, 0u);
+  } else {
+    const Group<TC> cg;
+    (void)settle<TC, L>(x, E, O, ov, c1, cg);
+  }
+  __syncwarp();
+  sq_get<TC, L>(r, low, g);
+#pragma unroll
+  for (int j = 0; j < L; ++j) {
+    const uint32_t h = __shfl_sync(kFull, x[j], g.c ? g.lane - TC : g.lane);
+    r[j] = g.c ? h : r[j];
+  }
 }
 
 }  // namespace hg

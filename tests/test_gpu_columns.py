@@ -111,3 +111,76 @@ def test_decrypt_full_range_and_non_units(edge_key, bits, dense):
         m = mp + p * ((mq - mp) * pow(p, -1, q) % q)
         want.append(m - n if m > n // 2 else m)
     assert key.decrypt_bn(hg.ints_to_limbs([c * R % n2 for c in odd], S)) == want
+
+
+def _randomness(key, rng, count):
+    r = rng.integers(0, 2 ** 32, (count, key.r_limbs), dtype=np.uint32)
+    r[0], r[1], r[2] = 0, 2 ** 32 - 1, 0
+    r[2, 0] = 1
+    r[3, :-1] = 0
+    return r
+
+
+@pytest.mark.parametrize("window", [1, 5, 8, 13])
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("bits", [1024, 2048, 3072])
+def test_encrypt_modes(gpu_ctx, edge_key, bits, dense, window):
+    """Encrypt, EncryptZero and Randomize byte for byte, over plaintexts up to
+    +-n/2 and randomness with zero, full and single digits."""
+    if window == 13 and bits != 2048:
+        pytest.skip("one wide window is enough")
+    _, n, h_s, _, _ = edge_key(bits, dense)
+    key = gpu_ctx.load_key(bits, n, h_s, table_window=window)
+    n2, S = n * n, key.ct_limbs
+    R = pow(2, 32 * S, n2)
+    rng = np.random.default_rng(window)
+    ms = [0, 1, -1, 2 ** 63 - 1, -(2 ** 63), n // 2, -(n // 2), 12345]
+    r = _randomness(key, rng, len(ms))
+    hr = [pow(h_s, v, n2) for v in hg.limbs_to_ints(r)]
+    want = [(1 + m * n) * h % n2 * R % n2 for m, h in zip(ms, hr)]
+    assert hg.limbs_to_ints(key.encrypt_bn(ms, r)) == want
+    assert hg.limbs_to_ints(key.encrypt(np.array(ms[:5]), r[:5])) == want[:5]
+    assert hg.limbs_to_ints(key.encrypt_zero(r)) == [h * R % n2 for h in hr]
+    edges = edge_values(n2, S)[:len(ms)]
+    got = key.randomize(hg.ints_to_limbs(edges, S), r)
+    assert hg.limbs_to_ints(got) == [c * h % n2 for c, h in zip(edges, hr)]
+    with pytest.raises(hg.HgError):
+        key.encrypt_bn([n // 2 + 1], r[:1])
+    with pytest.raises(hg.HgError):
+        key.randomize(hg.ints_to_limbs([n2], S), r[:1])
+    key.free()
+
+
+@pytest.mark.parametrize("bits", [1024, 2048, 3072])
+def test_encrypt_in_every_layout(edge_key, bits):
+    """A ciphertext does not depend on how many are encrypted with it: lengths
+    on both sides of the points where another layout runs."""
+    key, n, h_s, _, _ = edge_key(bits, True)
+    n2 = n * n
+    rng = np.random.default_rng(bits)
+    count = 21001
+    m = rng.integers(-(2 ** 63), 2 ** 63 - 1, count)
+    r = _randomness(key, rng, count)
+    ct = key.encrypt(m, r)
+    for i in (0, 1, 2, 3, 77, count - 1):
+        v = hg.limbs_to_ints(r[i])[0]
+        assert hg.limbs_to_ints(ct[i])[0] == pow(h_s, v, n2) * (1 + int(m[i]) * n) * pow(2, 2 * bits, n2) % n2
+    cfg = autotune.get_config(key)
+    for variant in (0, 1):
+        autotune.set_config(key, dict(cfg, variant=variant))
+        for length in (1, 3, 304, 305, 608, 609, 1217, 2500, 5001, 9729):
+            assert np.array_equal(key.encrypt(m[:length], r[:length]), ct[:length]), (variant, length)
+            assert np.array_equal(key.encrypt(m[-length:], r[-length:]), ct[-length:]), (variant, length)
+    autotune.set_config(key, cfg)
+
+
+def test_encrypt_with_a_base_that_is_no_unit(gpu_ctx, edge_key):
+    """h_s sharing a factor with n (never a key's) still encrypts by definition."""
+    _, n, h_s, p, q = edge_key(1024, False)
+    n2 = n * n
+    key = gpu_ctx.load_key(1024, n, h_s * p % n2, p, q, table_window=6)
+    r = _randomness(key, np.random.default_rng(0), 6)
+    ms = [0, 1, -1, 77, -5, 2 ** 40]
+    want = [pow(h_s * p, v, n2) * (1 + m * n) * pow(2, 2048, n2) % n2 for m, v in zip(ms, hg.limbs_to_ints(r))]
+    assert hg.limbs_to_ints(key.encrypt(np.array(ms), r)) == want
+    key.free()
