@@ -14,7 +14,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
-#include <type_traits>
 
 #include "paillier_ops.cuh"
 #include "sqmod.cuh"
@@ -31,46 +30,6 @@ template <int H>
 struct DecPrimes {
   uint32_t n[2][H];
 };
-
-// Vector words of a lane's slice in the odd-power table.
-template <int L>
-struct SliceVec {
-  using T = typename std::conditional<L % 4 == 0, uint4, uint2>::type;
-  static constexpr int kN = L % 4 == 0 ? L / 4 : L / 2;
-};
-
-// Odd-power table of a warp: [entry][vector][lane], so every load and store
-// of an entry is one contiguous run of the warp.
-template <int L>
-__device__ __forceinline__ void table_load(uint32_t (&x)[L], const uint32_t* tb, int e, uint32_t lane) {
-  using V = typename SliceVec<L>::T;
-  constexpr int kN = SliceVec<L>::kN, kW = sizeof(V) / 4;
-  const V* p = reinterpret_cast<const V*>(tb) + (size_t)e * kN * 32 + lane;
-#pragma unroll
-  for (int q = 0; q < kN; ++q) {
-    const V v = p[q * 32];
-    x[kW * q] = v.x;
-    x[kW * q + 1] = v.y;
-    if constexpr (kW == 4) {
-      x[kW * q + 2] = v.z;
-      x[kW * q + 3] = v.w;
-    }
-  }
-}
-
-template <int L>
-__device__ __forceinline__ void table_store(uint32_t* tb, int e, uint32_t lane, const uint32_t (&x)[L]) {
-  using V = typename SliceVec<L>::T;
-  constexpr int kN = SliceVec<L>::kN, kW = sizeof(V) / 4;
-  V* p = reinterpret_cast<V*>(tb) + (size_t)e * kN * 32 + lane;
-#pragma unroll
-  for (int q = 0; q < kN; ++q) {
-    if constexpr (kW == 4)
-      p[q * 32] = make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
-    else
-      p[q * 32] = make_uint2(x[2 * q], x[2 * q + 1]);
-  }
-}
 
 // One side of a warp's instances: digit 1 of c^(p-1) mod p^2, to
 // z[(2 i + side) H ..].  The exponent program and its table (2^(wd-1) odd

@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(128) k_sq_level(const __grid_constant__ KeyCon
 // chain, many with few.  2048 bits, window 12: 608 ciphertexts take 0.31 ms
 // with 16 lanes a chain (0.67 with 4), 4,864 take 0.99 ms with 4 (1.25 with 2
 // or 16), 131,072 take 23.5 ms with 2, 23.9 with 4 and 30.9 with 16.
-static double enc_cost(int H, int logtc, double warps) {
+double sq_pass_cost(int H, int logtc, double warps) {
   static const double lat[3][5] = {{6.8, 3.9, 2.7, 0, 1.8}, {0, 13.2, 7.2, 4.4, 3.3}, {0, 29, 15.3, 8.1, 5.4}};
   static const double thr[3][5] = {{4.67, 2.35, 1.35, 0, 0.56}, {0, 9.3, 4.76, 2.71, 1.54}, {0, 20.6, 10.7, 5.5, 3.4}};
   const int r = H == 32 ? 0 : H == 64 ? 1 : 2;
@@ -253,7 +253,7 @@ cudaError_t launch_sq_encrypt(int S, const KeyConst& kc, const EncArgs& a, uint3
     if ((H != 32 && l == 0) || (H == 32 && l == 3)) continue;
     const size_t ipw = (size_t)16 >> l;
     const double per = std::ceil((double)((count + ipw - 1) / ipw) / scheds);
-    const double cost = enc_cost(H, l, per);
+    const double cost = sq_pass_cost(H, l, per);
     if (cost < best_cost) {
       best_cost = cost;
       best = l;

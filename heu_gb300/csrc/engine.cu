@@ -538,7 +538,13 @@ void core_decrypt(KeyRec& k, Work& w, const uint32_t* ct, int64_t* m, uint8_t* o
   decrypt_crt(k, w, ct, m, ovf, mag, neg, count, hg::Codec{});
 }
 
-// out[i] = in[i]^-1 where sel == nullptr or sel[i] < 0, else in[i].
+// Nodes of a product tree over `count` leaves, all levels.
+size_t tree_nodes(size_t count) {
+  size_t total = 1;
+  for (size_t sz = count; sz > 1; sz = (sz + 1) / 2) total += sz;
+  return total;
+}
+
 // out[i] = in[i]^-1 where sel == nullptr or sel[i] < 0, else in[i]; every
 // step is in stream order (graph-capturable).  `task` must outlive the work.
 void core_inverse_async_raw(KeyRec& k, const uint32_t* in, const int64_t* sel, uint32_t* out, size_t count,
@@ -548,14 +554,11 @@ void core_inverse_async_raw(KeyRec& k, const uint32_t* in, const int64_t* sel, u
 void core_inverse_async(KeyRec& k, const uint32_t* in, const int64_t* sel, uint32_t* out, size_t count,
                         TreeBufs& tb, InvTask& task, uint32_t* errp, cudaStream_t st) {
   if (count == 0) return;
-  size_t padded = 1;
-  while (padded < count) padded <<= 1;
-  const size_t S = (size_t)k.S;
-  uint32_t* tr = tb.tree.ensure<uint32_t>(2 * padded * S * 4);
+  uint32_t* tr = tb.tree.ensure<uint32_t>(tree_nodes(count) * (size_t)k.S * 4);
   core_inverse_async_raw(k, in, sel, out, count, tr, task, errp, st);
 }
 
-// Same, on a caller-provided tree buffer of 2 * padded ciphertexts.  With
+// Same, on a caller-provided tree buffer of tree_nodes(count) ciphertexts.  With
 // inline_host the root is inverted by the calling thread after waiting for
 // the stream (the latency class of the server does this on its own
 // scheduler thread, so its batches never queue behind other streams' host
@@ -564,24 +567,21 @@ void core_inverse_async(KeyRec& k, const uint32_t* in, const int64_t* sel, uint3
 void core_inverse_async_raw(KeyRec& k, const uint32_t* in, const int64_t* sel, uint32_t* out, size_t count,
                             uint32_t* tr, InvTask& task, uint32_t* errp, cudaStream_t st, bool inline_host) {
   if (count == 0) return;
-  size_t padded = 1;
-  while (padded < count) padded <<= 1;
   const size_t S = (size_t)k.S;
-  // level l occupies [off_l, off_l + padded >> l)
-  std::vector<size_t> off;
+  // level l has size[l] nodes from off[l]; an odd one's last node has no sibling
+  std::vector<size_t> off, size;
   size_t total = 0;
-  for (size_t sz = padded;; sz >>= 1) {
+  for (size_t sz = count;; sz = (sz + 1) / 2) {
     off.push_back(total);
+    size.push_back(sz);
     total += sz;
     if (sz == 1) break;
   }
   task.N = &k.N;
   task.S = k.S;
-  cuda_check(hg::launch_tree_leaves(k.S, k.kc, in, sel, count, tr, padded, errp, st), "tree leaves");
-  for (size_t l = 0; l + 1 < off.size(); ++l) {
-    const size_t up = padded >> (l + 1);
-    cuda_check(hg::launch_tree_up(k.S, k.kc, tr + off[l] * S, tr + off[l + 1] * S, up, st), "tree up");
-  }
+  cuda_check(hg::launch_tree_leaves(k.S, k.kc, in, sel, count, tr, errp, st), "tree leaves");
+  for (size_t l = 0; l + 1 < off.size(); ++l)
+    cuda_check(hg::launch_tree_up(k.S, k.kc, tr + off[l] * S, size[l], tr + off[l + 1] * S, st), "tree up");
   uint32_t* root = tr + off.back() * S;
   cuda_check(cudaMemcpyAsync(task.root, root, S * 4, cudaMemcpyDeviceToHost, st), "D2H root");
   cuda_check(cudaMemcpyAsync(task.root + S, errp, 4, cudaMemcpyDeviceToHost, st), "D2H err");
@@ -592,10 +592,8 @@ void core_inverse_async_raw(KeyRec& k, const uint32_t* in, const int64_t* sel, u
     cuda_check(cudaLaunchHostFunc(st, inv_host_fn, &task), "host inversion");
   }
   cuda_check(cudaMemcpyAsync(root, task.z, S * 4, cudaMemcpyHostToDevice, st), "H2D inverse");
-  for (size_t l = off.size() - 1; l-- > 0;) {
-    const size_t up = padded >> (l + 1);
-    cuda_check(hg::launch_tree_down(k.S, k.kc, tr + off[l] * S, tr + off[l + 1] * S, up, st), "tree down");
-  }
+  for (size_t l = off.size() - 1; l-- > 0;)
+    cuda_check(hg::launch_tree_down(k.S, k.kc, tr + off[l] * S, size[l], tr + off[l + 1] * S, st), "tree down");
   cuda_check(hg::launch_tree_apply(k.S, k.kc, in, sel, tr, out, count, st), "tree apply");
 }
 
@@ -623,15 +621,28 @@ void core_inverse(KeyRec& k, Work& w, const uint32_t* in, const int64_t* sel, ui
   raise_task_status(w.task);
 }
 
-// sync_inverse = false leaves the inversion (k < 0) in stream order: the
-// caller resets w.task.status first and checks it after the stream drained.
-void core_mul(KeyRec& k, Work& w, const uint32_t* a, const int64_t* kk, const int64_t* host_k, uint32_t* out,
-              size_t count, bool sync_inverse = true) {
+// out[i] = a[i]^|k[i]|
+void mul_powers(KeyRec& k, Work& w, const uint32_t* a, const int64_t* kk, uint32_t* out, size_t count) {
+  if (count == 0) return;
+  if (k.kc.two_digit) {
+    const hg::MulPlan pl = hg::mul_plan(k.S, k.kc, k.wm, count);
+    uint32_t* scratch = w.scratch.ensure<uint32_t>(pl.scratch_words * 4);
+    cuda_check(hg::launch_sq_mul(k.S, k.kc, pl, a, kk, out, count, scratch, k.wm, w.errp(), w.ctrp(), w.stream),
+               "mul launch");
+    return;
+  }
   const size_t ntab = (size_t)1 << (k.wm - 1);
   const size_t inst = (size_t)k.grid_mul * hg::instances_per_block(k.S, k.kc.variant);
   uint32_t* scratch = w.scratch.ensure<uint32_t>(inst * ntab * k.S * 4);
   cuda_check(hg::launch_mul(k.S, k.kc, a, kk, out, count, scratch, k.wm, w.errp(), k.grid_mul, w.ctrp(), w.stream),
              "mul launch");
+}
+
+// sync_inverse = false leaves the inversion (k < 0) in stream order: the
+// caller resets w.task.status first and checks it after the stream drained.
+void core_mul(KeyRec& k, Work& w, const uint32_t* a, const int64_t* kk, const int64_t* host_k, uint32_t* out,
+              size_t count, bool sync_inverse = true) {
+  mul_powers(k, w, a, kk, out, count);
   bool any_neg = true;
   if (host_k) {
     any_neg = false;
@@ -903,7 +914,7 @@ bool build_sq_table(KeyRec& k) {
   }
   const BN ir = BN::invmod(rho1, n);  // rho^-1
   // entry (v0 | v1 / v0 rho) of v, given v0^-1 mod n
-  std::vector<uint32_t> hc(3 * (size_t)S + 6 * H);
+  std::vector<uint32_t> hc(6 * (size_t)S + 6 * H);
   auto entry = [&](size_t at, const BN& v, const BN& inv0) {
     (v % n).to_limbs(hc.data() + at, H);
     ((((digit1(v) * inv0) % n) * rho1) % n).to_limbs(hc.data() + at + H, H);
@@ -919,6 +930,13 @@ bool build_sq_table(KeyRec& k) {
   digit1(h).to_limbs(hc.data() + first + H, H);
   ih.to_limbs(hc.data() + first + 2 * H, H);
   ((ir * BN(1).shl(64)) % n).to_limbs(hc.data() + first + 3 * H, H);  // rho^2 / (2^(32 S) rho)
+  // digits of the scalar multiplication's constants
+  const size_t mul0 = 3 * (size_t)S + 6 * H;
+  const BN mulc[3] = {rho % N, BN(1).shl(32 * H + 96) % N, BN(1).shl(96 * H + 32) % N};
+  for (size_t j = 0; j < 3; ++j) {
+    (mulc[j] % n).to_limbs(hc.data() + mul0 + j * S, H);
+    digit1(mulc[j]).to_limbs(hc.data() + mul0 + j * S + H, H);
+  }
   uint32_t* d = k.sqconsts.ensure<uint32_t>(hc.size() * 4);
   cuda_check(cudaMemcpy(d, hc.data(), hc.size() * 4, cudaMemcpyHostToDevice), "upload consts");
   k.hn.assign(H, 0u);
@@ -928,6 +946,9 @@ bool build_sq_table(KeyRec& k) {
   kc.ie0 = d + first + 3 * H;
   kc.e1 = d + S;
   kc.rz = d + 2 * S;
+  kc.one = d + mul0;
+  kc.kin = d + mul0 + S;
+  kc.kout = d + mul0 + 2 * S;
   kc.rho2 = d + 3 * S;
   kc.nrho2 = d + 3 * S + H;
   kc.hn = k.hn.data();
@@ -2528,8 +2549,7 @@ void batch_build(hg_batch& b) {
   b.pin_err.ensure<uint32_t>(4);
   // size the inversion trees now so nothing allocates during a capture
   for (auto& inv : b.invs) {
-    const size_t padded = padded_pow2(b.jobs[inv->job].count);
-    inv->bufs.tree.ensure<uint32_t>((2 * padded) * (size_t)inv->key->S * 4);
+    inv->bufs.tree.ensure<uint32_t>(tree_nodes(b.jobs[inv->job].count) * (size_t)inv->key->S * 4);
   }
   b.dirty = false;
 }
@@ -2626,11 +2646,7 @@ int hg_autotune(hg_ctx* ctx, int key_id, size_t calib, hg_key_config* best, doub
         c.mul_window = wm;
         apply_config(*k, c);
         const double tm = timed([&] {
-          const size_t inst = (size_t)k->grid_mul * hg::instances_per_block(k->S, k->kc.variant);
-          uint32_t* scratch = w.scratch.ensure<uint32_t>(inst * ((size_t)1 << (k->wm - 1)) * k->S * 4);
-          cuda_check(hg::launch_mul(k->S, k->kc, dct, dk, dout, n, scratch, k->wm, w.errp(), k->grid_mul, w.ctrp(),
-                                    w.stream),
-                     "mul launch");
+          mul_powers(*k, w, dct, dk, dout, n);
         });
         if (te + tm < best_nn) {
           best_nn = te + tm;

@@ -233,55 +233,58 @@ __global__ void __launch_bounds__(kBlock) k_reduce_tree(KeyConst kc, const uint3
 // Product tree for batch inversion (Montgomery's simultaneous-inversion
 // trick arranged as a tree): leaves, up-sweep, root fix, down-sweep, apply.
 // ---------------------------------------------------------------------------
+// A level of c nodes has ceil(c / 2) parents; an odd level's last node is its
+// parent's only child and goes up and down unchanged.
 template <int TPI, int L>
 __global__ void __launch_bounds__(kBlock) k_tree_leaves(KeyConst kc, const uint32_t* __restrict__ in,
                                                         const int64_t* __restrict__ sel, size_t count,
-                                                        uint32_t* __restrict__ leaves, size_t padded,
-                                                        uint32_t* err) {
+                                                        uint32_t* __restrict__ leaves, uint32_t* err) {
   constexpr int S = TPI * L;
-  const Group<TPI> g;
-  const size_t inst = ((size_t)blockIdx.x * kBlock + threadIdx.x) / TPI;
-  const size_t wfirst = ((size_t)blockIdx.x * kBlock + (threadIdx.x & ~31u)) / TPI;
-  if (wfirst >= padded) return;
-  const size_t i = inst < count ? inst : count - 1;
+  HG_INSTANCE_PROLOGUE(count)
   uint32_t A[L], N[L], one[L];
   load_slice<L>(A, in + i * S + g.t * L);
   load_slice<L>(N, kc.N + g.t * L);
   load_slice<L>(one, kc.R1 + g.t * L);
-  const bool use = inst < count && (sel == nullptr || sel[i] < 0);
+  const bool use = sel == nullptr || sel[i] < 0;
   check_ct<TPI, L>(A, N, use, g, err);
   select_slice<L>(A, use, A, one);
-  if (inst < padded) store_slice<L>(leaves + inst * S + g.t * L, A);
+  if (active) store_slice<L>(leaves + i * S + g.t * L, A);
 }
 
 template <int TPI, int L>
 __global__ void __launch_bounds__(kBlock) k_tree_up(KeyConst kc, const uint32_t* __restrict__ lower,
-                                                    uint32_t* __restrict__ upper, size_t upper_count) {
+                                                    size_t lower_count, uint32_t* __restrict__ upper) {
   constexpr int S = TPI * L;
+  const size_t upper_count = (lower_count + 1) / 2;
   HG_INSTANCE_PROLOGUE(upper_count)
-  uint32_t N[L], A[L], B[L];
+  const bool pair = 2 * i + 1 < lower_count;
+  uint32_t N[L], A[L], B[L], r[L];
   load_slice<L>(N, kc.N + g.t * L);
   load_slice<L>(A, lower + (2 * i) * S + g.t * L);
-  load_slice<L>(B, lower + (2 * i + 1) * S + g.t * L);
-  mont_mul<TPI, L>(A, A, B, N, kc.np, g);
-  if (active) store_slice<L>(upper + i * S + g.t * L, A);
+  load_slice<L>(B, lower + (2 * i + (pair ? 1 : 0)) * S + g.t * L);
+  mont_mul<TPI, L>(r, A, B, N, kc.np, g);
+  select_slice<L>(r, pair, r, A);
+  if (active) store_slice<L>(upper + i * S + g.t * L, r);
 }
 
 template <int TPI, int L>
-__global__ void __launch_bounds__(kBlock) k_tree_down(KeyConst kc, uint32_t* __restrict__ lower,
-                                                      const uint32_t* __restrict__ upper_inv, size_t upper_count) {
+__global__ void __launch_bounds__(kBlock) k_tree_down(KeyConst kc, uint32_t* __restrict__ lower, size_t lower_count,
+                                                      const uint32_t* __restrict__ upper_inv) {
   constexpr int S = TPI * L;
+  const size_t upper_count = (lower_count + 1) / 2;
   HG_INSTANCE_PROLOGUE(upper_count)
-  uint32_t N[L], U[L], A[L], B[L], ra[L], rb[L];
+  const bool pair = 2 * i + 1 < lower_count;
+  uint32_t N[L], U[L], A[L], B[L], ra[L];
   load_slice<L>(N, kc.N + g.t * L);
   load_slice<L>(U, upper_inv + i * S + g.t * L);
   load_slice<L>(A, lower + (2 * i) * S + g.t * L);
-  load_slice<L>(B, lower + (2 * i + 1) * S + g.t * L);
+  load_slice<L>(B, lower + (2 * i + (pair ? 1 : 0)) * S + g.t * L);
   mont_mul<TPI, L>(ra, U, B, N, kc.np, g);  // inverse of A
-  mont_mul<TPI, L>(rb, U, A, N, kc.np, g);  // inverse of B
+  select_slice<L>(ra, pair, ra, U);
+  mont_mul<TPI, L>(A, U, A, N, kc.np, g);  // inverse of B
   if (active) {
     store_slice<L>(lower + (2 * i) * S + g.t * L, ra);
-    store_slice<L>(lower + (2 * i + 1) * S + g.t * L, rb);
+    if (pair) store_slice<L>(lower + (2 * i + 1) * S + g.t * L, A);
   }
 }
 
@@ -591,25 +594,23 @@ int reduce_tree_chunk(int S, size_t count, int sms) {
 }
 
 cudaError_t launch_tree_leaves(int S, const KeyConst& kc, const uint32_t* in, const int64_t* sel, size_t count,
-                               uint32_t* leaves, size_t padded, uint32_t* err, cudaStream_t st) {
+                               uint32_t* leaves, uint32_t* err, cudaStream_t st) {
   HG_DISPATCH_S0(S,
-                 k_tree_leaves<TPI, L><<<blocks_for(padded, TPI), kBlock, 0, st>>>(kc, in, sel, count, leaves,
-                                                                                   padded, err));
+                 k_tree_leaves<TPI, L><<<blocks_for(count, TPI), kBlock, 0, st>>>(kc, in, sel, count, leaves, err));
   return counted();
 }
 
-cudaError_t launch_tree_up(int S, const KeyConst& kc, const uint32_t* lower, uint32_t* upper, size_t upper_count,
+cudaError_t launch_tree_up(int S, const KeyConst& kc, const uint32_t* lower, size_t lower_count, uint32_t* upper,
                            cudaStream_t st) {
-  HG_DISPATCH_S0(S,
-                 k_tree_up<TPI, L><<<blocks_for(upper_count, TPI), kBlock, 0, st>>>(kc, lower, upper, upper_count));
+  HG_DISPATCH_S0(S, k_tree_up<TPI, L><<<blocks_for((lower_count + 1) / 2, TPI), kBlock, 0, st>>>(kc, lower, lower_count,
+                                                                                             upper));
   return counted();
 }
 
-cudaError_t launch_tree_down(int S, const KeyConst& kc, uint32_t* lower, const uint32_t* upper_inv,
-                             size_t upper_count, cudaStream_t st) {
-  HG_DISPATCH_S0(S,
-                 k_tree_down<TPI, L><<<blocks_for(upper_count, TPI), kBlock, 0, st>>>(kc, lower, upper_inv,
-                                                                                      upper_count));
+cudaError_t launch_tree_down(int S, const KeyConst& kc, uint32_t* lower, size_t lower_count,
+                             const uint32_t* upper_inv, cudaStream_t st) {
+  HG_DISPATCH_S0(S, k_tree_down<TPI, L><<<blocks_for((lower_count + 1) / 2, TPI), kBlock, 0, st>>>(
+                        kc, lower, lower_count, upper_inv));
   return counted();
 }
 

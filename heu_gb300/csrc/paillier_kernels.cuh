@@ -45,6 +45,11 @@ struct KeyConst {
   const uint32_t* rho2;   // rho^2 mod n   (H limbs)
   const uint32_t* nrho2;  // -rho^2 mod n  (H limbs)
   const uint32_t* hn;     // n on the host (H limbs)
+  // two-digit scalar multiplication (sq_mul.cuh), digits of constants modulo
+  // n^2 (S limbs each): rho, rho^3 / 2^(32 S) into the form, 2^(32 S) rho out
+  const uint32_t* one;
+  const uint32_t* kin;
+  const uint32_t* kout;
 };
 
 // Secret-key constants for CRT decryption.  Index 0 = p side, 1 = q side.
@@ -86,6 +91,10 @@ struct OuConst {
   int wd;                 // window bits
   int Sp;                 // 32-bit limbs of the p^2 arithmetic
 };
+
+// Table entries of a warp's scalar multiplication (sq_mul.cuh): the powers 0 ..
+// 2^wm - 1, then the constants into and out of the form of radix rho.
+__host__ __device__ constexpr int mul_slots(int wm) { return (1 << wm) + 2; }
 
 // Exponent-program opcodes (one Montgomery multiplication per step).
 constexpr uint16_t kOpSquare = 0xFFFFu;
@@ -143,6 +152,19 @@ cudaError_t launch_add_plain(int S, const KeyConst& kc, const uint32_t* a, const
 cudaError_t launch_mul(int S, const KeyConst& kc, const uint32_t* a, const int64_t* k, uint32_t* out,
                        size_t count, uint32_t* scratch, int wm, uint32_t* err, int grid, unsigned long long* ctr,
                        cudaStream_t st);
+// Mul of two-digit keys (mul_kernels.cu) over mul_plan's scratch.
+struct MulPlan {
+  int logtc = 1;  // log2 of the lanes per chain
+  int warps = 0;
+  size_t scratch_words = 0;
+};
+MulPlan mul_plan(int S, const KeyConst& kc, int wm, size_t count);
+cudaError_t launch_sq_mul(int S, const KeyConst& kc, const MulPlan& pl, const uint32_t* a, const int64_t* k,
+                          uint32_t* out, size_t count, uint32_t* scratch, int wm, uint32_t* err,
+                          unsigned long long* ctr, cudaStream_t st);
+// Time (us) of a pass modulo an H-limb n's square with `warps` warps of a
+// layout on every scheduler (encrypt_kernels.cu).
+double sq_pass_cost(int H, int logtc, double warps);
 // Mul by multi-limb scalar magnitudes (el limbs each), window wb (1..8);
 // persistent grid of `grid` blocks (resident_blocks_mul_bn) with a scratch of
 // grid * instances_per_block(S, 0) * 2^(wb-1) * S limbs.
@@ -202,11 +224,11 @@ cudaError_t launch_reduce(int S, const KeyConst& kc, const uint32_t* in, size_t 
                           uint32_t* out, uint32_t* err, cudaStream_t st);
 // product tree for batch inversion
 cudaError_t launch_tree_leaves(int S, const KeyConst& kc, const uint32_t* in, const int64_t* sel, size_t count,
-                               uint32_t* leaves, size_t padded, uint32_t* err, cudaStream_t st);
-cudaError_t launch_tree_up(int S, const KeyConst& kc, const uint32_t* lower, uint32_t* upper, size_t upper_count,
+                               uint32_t* leaves, uint32_t* err, cudaStream_t st);
+cudaError_t launch_tree_up(int S, const KeyConst& kc, const uint32_t* lower, size_t lower_count, uint32_t* upper,
                            cudaStream_t st);
-cudaError_t launch_tree_down(int S, const KeyConst& kc, uint32_t* lower, const uint32_t* upper_inv,
-                             size_t upper_count, cudaStream_t st);
+cudaError_t launch_tree_down(int S, const KeyConst& kc, uint32_t* lower, size_t lower_count,
+                             const uint32_t* upper_inv, cudaStream_t st);
 cudaError_t launch_tree_apply(int S, const KeyConst& kc, const uint32_t* in, const int64_t* sel,
                               const uint32_t* leaves_inv, uint32_t* out, size_t count, cudaStream_t st);
 // fixed-base table construction

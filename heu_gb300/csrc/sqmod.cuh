@@ -26,6 +26,8 @@
 // array of L words: registers, or with TC = 1 the kernel's constant bank,
 // which frees L registers.
 #pragma once
+#include <type_traits>
+
 #include "mont.cuh"
 
 namespace hg {
@@ -283,6 +285,47 @@ __device__ __forceinline__ void sq_redc(uint32_t (&z)[L], const uint32_t (&x)[L]
   }
   sq_redc_step<TC, L>(E, O, ov, c1, n, np, 0u, g);
   sq_settle<TC, L>(z, O, E, c1, n, g);
+}
+
+// ---- tables of a warp in global scratch ---------------------------------------
+// Vector words of a lane's slice.
+template <int L>
+struct SliceVec {
+  using T = typename std::conditional<L % 4 == 0, uint4, uint2>::type;
+  static constexpr int kN = L % 4 == 0 ? L / 4 : L / 2;
+};
+
+// A warp's table: [entry][vector][lane], so the load or store of one entry by
+// all lanes is one contiguous run.
+template <int L>
+__device__ __forceinline__ void table_load(uint32_t (&x)[L], const uint32_t* tb, int e, uint32_t lane) {
+  using V = typename SliceVec<L>::T;
+  constexpr int kN = SliceVec<L>::kN, kW = sizeof(V) / 4;
+  const V* p = reinterpret_cast<const V*>(tb) + (size_t)e * kN * 32 + lane;
+#pragma unroll
+  for (int q = 0; q < kN; ++q) {
+    const V v = p[q * 32];
+    x[kW * q] = v.x;
+    x[kW * q + 1] = v.y;
+    if constexpr (kW == 4) {
+      x[kW * q + 2] = v.z;
+      x[kW * q + 3] = v.w;
+    }
+  }
+}
+
+template <int L>
+__device__ __forceinline__ void table_store(uint32_t* tb, int e, uint32_t lane, const uint32_t (&x)[L]) {
+  using V = typename SliceVec<L>::T;
+  constexpr int kN = SliceVec<L>::kN, kW = sizeof(V) / 4;
+  V* p = reinterpret_cast<V*>(tb) + (size_t)e * kN * 32 + lane;
+#pragma unroll
+  for (int q = 0; q < kN; ++q) {
+    if constexpr (kW == 4)
+      p[q * 32] = make_uint4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+    else
+      p[q * 32] = make_uint2(x[2 * q], x[2 * q + 1]);
+  }
 }
 
 // ---- digit helpers over one chain -------------------------------------------

@@ -184,3 +184,64 @@ def test_encrypt_with_a_base_that_is_no_unit(gpu_ctx, edge_key):
     want = [pow(h_s * p, v, n2) * (1 + m * n) * pow(2, 2048, n2) % n2 for m, v in zip(ms, hg.limbs_to_ints(r))]
     assert hg.limbs_to_ints(key.encrypt(np.array(ms), r)) == want
     key.free()
+
+
+def _scalars(rng, count):
+    k = rng.integers(-(2 ** 63), 2 ** 63 - 1, count)
+    k[: min(count, 14)] = [0, 1, -1, 2, -2, 2 ** 63 - 1, -(2 ** 63), 15, 16, 17, -16, 2 ** 32, 2 ** 60, -3][:count]
+    return k
+
+
+@pytest.mark.parametrize("window", [2, 4, 6])
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("bits", [1024, 2048, 3072])
+def test_mul_windows(edge_key, bits, dense, window):
+    """Scalars of every length (a warp's windows follow its longest) on edge
+    ciphertexts, byte for byte; 15 of them leave a ragged warp and an odd node
+    on every level of the inverse's tree."""
+    key, n, h_s, _, _ = edge_key(bits, dense)
+    n2, S = n * n, key.ct_limbs
+    R = pow(2, 32 * S, n2)
+    rng = np.random.default_rng(window)
+    k = _scalars(rng, 15)
+    units = [pow(h_s, 3 + i, n2) * R % n2 for i in range(len(k) - 4)] + [1, 2, n2 - 1, n2 - 2]
+    cfg = autotune.get_config(key)
+    autotune.set_config(key, dict(cfg, mul_window=window))
+    got = hg.limbs_to_ints(key.mul(hg.ints_to_limbs(units, S), k))
+    small = hg.limbs_to_ints(key.mul(hg.ints_to_limbs(units, S), k % 5))
+    autotune.set_config(key, cfg)
+    rinv = pow(R, -1, n2)
+    assert got == [pow(c * rinv % n2, int(e), n2) * R % n2 for c, e in zip(units, k)]
+    assert small == [pow(c * rinv % n2, int(e), n2) * R % n2 for c, e in zip(units, k % 5)]
+    # numbers that are no units, and no ciphertexts at all
+    none = [v for v in edge_values(n2, S)]
+    pos = np.abs(k[: len(none)] // 2)
+    assert hg.limbs_to_ints(key.mul(hg.ints_to_limbs(none, S), pos)) == [
+        pow(c * rinv % n2, int(e), n2) * R % n2 for c, e in zip(none, pos)]
+    with pytest.raises(hg.HgError):
+        key.mul(hg.ints_to_limbs([n2], S), [3])
+
+
+@pytest.mark.parametrize("bits", [1024, 2048, 3072])
+def test_mul_in_every_layout(edge_key, bits):
+    """A product does not depend on how many there are: lengths on both sides
+    of the points where another layout runs, with signed scalars (every length
+    another inverse tree)."""
+    key, n, h_s, _, _ = edge_key(bits, False)
+    n2, S = n * n, key.ct_limbs
+    R = pow(2, 32 * S, n2)
+    rinv = pow(R, -1, n2)
+    rng = np.random.default_rng(bits)
+    count = 10007
+    k = _scalars(rng, count)
+    ct = key.encrypt(rng.integers(-(2 ** 40), 2 ** 40, count), _randomness(key, rng, count))
+    whole = key.mul(ct, k)
+    for i in (0, 6, 7, 20, 5000, count - 1):
+        c = hg.limbs_to_ints(ct[i])[0] * rinv % n2
+        assert hg.limbs_to_ints(whole[i])[0] == pow(c, int(k[i]), n2) * R % n2
+    cfg = autotune.get_config(key)
+    for variant in (0, 1):
+        autotune.set_config(key, dict(cfg, variant=variant))
+        for length in (1, 2, 3, 9, 301, 609, 1217, 2433, 4865, count):
+            assert np.array_equal(key.mul(ct[:length], k[:length]), whole[:length]), (variant, length)
+    autotune.set_config(key, cfg)
