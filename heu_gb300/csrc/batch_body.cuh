@@ -18,15 +18,18 @@
 
 #include "batch.cuh"
 #include "paillier_ops.cuh"
+#include "sq_decrypt.cuh"
 #include "sq_encrypt.cuh"
+#include "sq_mul.cuh"
 
 namespace hg {
 
 namespace batch_detail {
 constexpr int kBlock = 128;
 constexpr int kWarps = kBlock / 32;
-// Shared words of a warp: 32 limbs a lane of the decryption's hand-off (up to
-// 24 limbs a lane), 5 x 16 of the encryption's areas (up to 16, 32 and 6).
+// Shared words of a warp: 80 a limb of a lane for the encryption's areas (up to
+// 16, 32 and 6 limbs a lane), at least 48 a limb and 8 a limb of the prime for
+// the decryption's.
 template <int V>
 constexpr int kAreaWords = V == 1 ? 80 * 32 : V == 0 ? 80 * 16 : 768;
 }  // namespace batch_detail
@@ -39,18 +42,31 @@ __device__ __forceinline__ void run_tile(const BatchJob& job, const BatchTile& t
   const size_t end = (size_t)tile.start + tile.count;
   if (job.op == kBatchDecrypt) {
     constexpr int SP = S / 2;
-    constexpr int TP = tp_for(SP, V), LP = SP / TP;
+    // a group of TP lanes per side, TP / 2 a chain; both sides of a
+    // ciphertext in neighbouring groups
+    constexpr int TP = tp_for(SP, V), TC = TP / 2, LC = SP / TP, H = SP / 2;
     constexpr int UPW = 32 / (2 * TP);
-    const Group<TP> g;
-    const int side = (lane / TP) & 1;
-    const int unit_w = lane / (2 * TP);
-    const int ntab = 1 << (job.sc.wd - 1);
-    uint32_t* tb = ws + ((size_t)unit_w * 2 + side) * (size_t)ntab * SP + g.t * LP;
+    const SqLanes<TC, LC> g;
+    const int side = g.iw & 1, unit_w = g.iw >> 1;
+    uint32_t* zs = ysm + 2 * SqLanes<TC, LC>::kDigit;
+    uint32_t* mm = zs + UPW * 2 * H;
+    static_assert(2 * SqLanes<TC, LC>::kDigit + UPW * 2 * H + 4 * 2 * H <= batch_detail::kAreaWords<V>, "area");
     for (size_t wbase = tile.start; wbase < end; wbase += UPW) {
       const size_t inst = wbase + unit_w;
       const bool active = inst < end;
-      decrypt_one<TP, LP>(job.kc, job.sc, (const uint32_t*)job.in0, active ? inst : end - 1, active, side, tb,
-                          ysm + unit_w * 2 * SP, (int64_t*)job.out, (uint8_t*)job.aux, nullptr, nullptr, g, err);
+      __syncwarp();
+      dec_pow_fixed<TC, LC>(job.kc, job.sc, side, (const uint32_t*)job.in0, active ? inst : end - 1, active, ws, ysm,
+                            zs + g.iw * H, err, g);
+      __syncwarp();
+      // 8 lanes a ciphertext
+#pragma unroll 1
+      for (int u0 = 0; u0 < UPW; u0 += 4) {
+        const int u = min(u0 + lane / 8, UPW - 1);
+        const bool mine = u0 + lane / 8 < UPW && wbase + u < end;
+        dec_tail<H / 8>(job.kc, job.sc, zs + u * 2 * H, mine ? wbase + u : end - 1, mine, mm + (lane / 8) * 2 * H,
+                        (int64_t*)job.out, (uint8_t*)job.aux, nullptr, nullptr, Codec{});
+        __syncwarp();
+      }
     }
     return;
   }
@@ -87,6 +103,17 @@ __device__ __forceinline__ void run_tile(const BatchJob& job, const BatchTile& t
       add_one<TPI, L>(job.kc, (const uint32_t*)job.in0, (const uint32_t*)job.in1, (uint32_t*)job.out,
                       active ? inst : end - 1, active, N, g, err);
     }
+  } else if (job.op == kBatchMul && job.kc.two_digit) {
+    const SqLanes<TPI / 2, L> sg;
+    uint32_t n[L];
+    load_slice<L>(n, job.kc.n + sg.t * L);
+    for (size_t wbase = tile.start; wbase < end; wbase += IPW) {
+      const size_t inst = wbase + lane_inst;
+      const bool active = inst < end;
+      __syncwarp();
+      sq_mul<TPI / 2, L>(n, job.kc, (const uint32_t*)job.in0, (const int64_t*)job.in1, (uint32_t*)job.out,
+                         active ? inst : end - 1, active, ws, job.wm, ysm, err, sg);
+    }
   } else if (job.op == kBatchMul) {
     const int ntab = 1 << (job.wm - 1);
     uint32_t* tb = ws + (size_t)lane_inst * ntab * S + g.t * L;
@@ -99,8 +126,10 @@ __device__ __forceinline__ void run_tile(const BatchJob& job, const BatchTile& t
   }
 }
 
+// Four blocks per SM in the layouts that fit them: the server splits an SM's
+// blocks between its regular and its short batches.
 template <int V>
-__global__ void __launch_bounds__(batch_detail::kBlock) k_batch(const BatchJob* __restrict__ jobs,
+__global__ void __launch_bounds__(batch_detail::kBlock, V == 1 ? 1 : 4) k_batch(const BatchJob* __restrict__ jobs,
                                                   const BatchTile* __restrict__ tiles, uint32_t ntiles,
                                                   uint32_t* __restrict__ counter, uint32_t* __restrict__ scratch,
                                                   size_t warp_words, uint32_t* err) {

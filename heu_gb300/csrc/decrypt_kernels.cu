@@ -15,8 +15,7 @@
 #include <atomic>
 #include <cmath>
 
-#include "paillier_ops.cuh"
-#include "sqmod.cuh"
+#include "sq_decrypt.cuh"
 
 namespace hg {
 
@@ -79,15 +78,7 @@ __device__ __forceinline__ void dec_pow_side(const Mod& n, const KeyConst& kc, c
     }
     if (s < ntab) table_store<L>(tb, s == 0 ? ntab : s, g.lane, x);
   }
-  sq_redc<TC, L>(x, x, n, np, g);
-  // digit 0 is 1, or a multiple of p where p divides c: such a c decrypts as
-  // it always did, through the value that stands for it
-  uint32_t any = x[0] ^ (g.t == 0 ? 1u : 0u);
-#pragma unroll
-  for (int j = 1; j < L; ++j) any |= x[j];
-  const uint32_t mask = (1u << TC) - 1u;
-  const bool zero = ((__ballot_sync(kFull, any != 0u) >> g.base) & mask) != 0u;
-  if (zero) load_slice<L>(x, sc.vz[side] + g.t * L);
+  dec_digit<TC, L>(x, sc, side, n, np, g);
   if (active && g.c == 1) store_slice<L>(z + (2 * i + side) * H + g.t * L, x);
 }
 
@@ -128,10 +119,7 @@ __global__ void __launch_bounds__(32, dec_min_blocks(L))
   }
 }
 
-// m_p = z_p c1_p + c2_p mod p, the same for q, then the CRT combination
-//   h = (m_q - m_p) p^-1 mod q, m = m_p + p h
-// and the sign fold m > n/2 => m - n (decryptor.cc:49-52).  8 lanes per
-// ciphertext; under 1% of the decryption.
+// dec_tail over all ciphertexts of a chunk; under 1% of the decryption.
 template <int LT>
 __global__ void __launch_bounds__(128) k_dec_tail(const __grid_constant__ KeyConst kc,
                                                   const __grid_constant__ SecConst sc,
@@ -139,88 +127,12 @@ __global__ void __launch_bounds__(128) k_dec_tail(const __grid_constant__ KeyCon
                                                   int64_t* __restrict__ out_i64, uint8_t* __restrict__ out_ovf,
                                                   uint32_t* __restrict__ out_mag, uint8_t* __restrict__ out_neg,
                                                   const __grid_constant__ Codec cd, size_t first) {
-  constexpr int TP = 8, H = TP * LT, W = 2 * LT;
-  __shared__ __align__(16) uint32_t mms[128 / TP][2 * H];
-  const Group<TP> g;
-  const size_t inst = ((size_t)blockIdx.x * 128 + threadIdx.x) / TP;
+  constexpr int H = 8 * LT;
+  __shared__ __align__(16) uint32_t mm[16][2 * H];
+  const size_t inst = ((size_t)blockIdx.x * 128 + threadIdx.x) / 8;
   const bool active = inst < count;
   const size_t u = active ? inst : count - 1;
-  const size_t i = first + u;
-  uint32_t* mm = mms[threadIdx.x / TP];
-  uint32_t P[LT], Q[LT], a[LT], b[LT], mp[LT], mq[LT];
-  load_slice<LT>(P, sc.P[0] + g.t * LT);
-  load_slice<LT>(Q, sc.P[1] + g.t * LT);
-  load_slice<LT>(a, z + (2 * u) * H + g.t * LT);
-  load_slice<LT>(b, sc.c1[0] + g.t * LT);
-  mont_mul<TP, LT>(mp, a, b, P, sc.np1[0], g);
-  load_slice<LT>(b, sc.c2[0] + g.t * LT);
-  mod_add<TP, LT>(mp, mp, b, P, g);
-  load_slice<LT>(a, z + (2 * u + 1) * H + g.t * LT);
-  load_slice<LT>(b, sc.c1[1] + g.t * LT);
-  mont_mul<TP, LT>(mq, a, b, Q, sc.np1[1], g);
-  load_slice<LT>(b, sc.c2[1] + g.t * LT);
-  mod_add<TP, LT>(mq, mq, b, Q, g);
-  // m_p mod q (p < 2q), then h
-  reduce_once<TP, LT>(a, mp, 0u, Q, g);
-  mod_sub<TP, LT>(mq, mq, a, Q, g);
-  load_slice<LT>(b, sc.pinvqR + g.t * LT);
-  mont_mul<TP, LT>(mq, mq, b, Q, sc.np1[1], g);
-  // m = m_p + p h: rows of p, the lowest limb leaves in every step
-  {
-    uint32_t E[LT], O[LT], T[LT], ov = 0u, c1 = 0u;
-#pragma unroll
-    for (int j = 0; j < LT; ++j) {
-      E[j] = mp[j];
-      O[j] = 0u;
-    }
-#pragma unroll 1
-    for (int owner = 0; owner < TP; ++owner) {
-#pragma unroll
-      for (int j = 0; j < LT; j += 2) {
-        row_mac<LT>(E, O, ov, c1, P, __shfl_sync(kFull, mq[j], owner, TP));
-        if (g.t == 0) mm[owner * LT + j] = E[0];
-        shift_limb<TP, LT>(E, ov, c1, g);
-        row_mac<LT>(O, E, ov, c1, P, __shfl_sync(kFull, mq[j + 1], owner, TP));
-        if (g.t == 0) mm[owner * LT + j + 1] = O[0];
-        shift_limb<TP, LT>(O, ov, c1, g);
-      }
-    }
-    (void)settle<TP, LT>(T, E, O, ov, c1, g);
-    store_slice<LT>(mm + H + g.t * LT, T);
-  }
-  __syncwarp();
-  uint32_t M[W], X[W], D[W];
-  load_slice<W>(M, mm + g.t * W);
-  load_slice<W>(X, kc.nhalf + g.t * W);
-  const bool gt = sub_full<TP, W>(D, X, M, g) != 0u;
-  load_slice<W>(X, kc.n + g.t * W);
-  (void)sub_full<TP, W>(D, X, M, g);
-  select_slice<W>(M, gt, D, M);
-  __syncwarp();
-  store_slice<W>(mm + g.t * W, M);
-  __syncwarp();
-  if (cd.kind != kCodecNone) {
-    if (active && g.t == 0) decode_plain<2 * H>(cd, mm, gt, i, out_i64, out_ovf);
-    return;
-  }
-  if (out_mag) {
-    if (active) store_slice<W>(out_mag + i * (2 * H) + g.t * W, M);
-    if (active && g.t == 0) out_neg[i] = gt ? 1 : 0;
-  }
-  if (out_i64) {
-    uint32_t high = 0u;
-#pragma unroll
-    for (int j = 0; j < W; ++j)
-      if (g.t != 0 || j >= 2) high |= M[j];
-    const uint32_t B = __ballot_sync(kFull, high != 0u);
-    bool fits = ((B >> g.base) & 0xffu) == 0u;
-    if (active && g.t == 0) {
-      const uint64_t mag = (uint64_t)M[0] | ((uint64_t)M[1] << 32);
-      fits = fits && (gt ? mag <= (1ull << 63) : mag < (1ull << 63));
-      out_i64[i] = (int64_t)(gt ? (uint64_t)0 - mag : mag);
-      if (out_ovf) out_ovf[i] = fits ? 0 : 1;
-    }
-  }
+  dec_tail<LT>(kc, sc, z + u * 2 * H, first + u, active, mm[threadIdx.x / 8], out_i64, out_ovf, out_mag, out_neg, cd);
 }
 
 // Layouts by (limbs of a prime, log2 of the lanes per chain).

@@ -174,7 +174,7 @@ struct KeyRec {
   int S = 0, Sp = 0, H = 0;
   bool secret = false;
   BN n, N, hs, p, q;
-  DevBuf consts, sconsts, table, progs;
+  DevBuf consts, sconsts, table, progs, fprogs;
   DevBuf sqconsts;            // two-digit encryption: e0 e1 rz (S each), rho2, nrho2 (H each)
   std::vector<uint32_t> hn;   // n (S/2 limbs)
   hg::KeyConst kc{};
@@ -1036,20 +1036,12 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
     // mod pr the power is 1 + (pr-1) n, so L is -n/pr mod pr
     const BN hp = BN::invmod(k->p - k->q % k->p, k->p), hq = BN::invmod(k->q - k->p % k->q, k->q);
     const BN pinvq = BN::invmod(k->p, k->q);
-    // p2 q2 (Sp) | p q hR_p hR_q inv2_p inv2_q pinvqR c1_p c1_q c2_p c2_q vz_p vz_q (H)
-    std::vector<uint32_t> hs2(2 * (size_t)Sp + 13 * (size_t)H);
+    // p q pinvqR c1_p c1_q c2_p c2_q vz_p vz_q (H) | one_p one_q (Sp)
+    std::vector<uint32_t> hs2(2 * (size_t)Sp + 9 * (size_t)H);
     auto put2 = [&](size_t at, const BN& v, size_t limbs) { v.to_limbs(hs2.data() + at, limbs); };
-    put2(0, p2, Sp);
-    put2(Sp, q2, Sp);
-    size_t o = 2 * (size_t)Sp;
-    put2(o, k->p, H);
-    put2(o + H, k->q, H);
-    put2(o + 2 * H, (hp * R1h) % k->p, H);
-    put2(o + 3 * H, (hq * R1h) % k->q, H);
-    const BN inv2[2] = {BN::invmod(k->p, R1h), BN::invmod(k->q, R1h)};
-    put2(o + 4 * H, inv2[0], H);
-    put2(o + 5 * H, inv2[1], H);
-    put2(o + 6 * H, (pinvq * R1h) % k->q, H);
+    put2(0, k->p, H);
+    put2(H, k->q, H);
+    put2(2 * H, (pinvq * R1h) % k->q, H);
     for (int sd = 0; sd < 2; ++sd) {
       const BN &pr = sd ? k->q : k->p, &pr2 = sd ? q2 : p2, &h = sd ? hq : hp;
       auto neg = [&](const BN& v) { return v.is_zero() ? v : pr - v; };  // v < pr
@@ -1057,10 +1049,14 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
       // its power is 1 + d pr with d = -64 (2^(pr-1) - 1) / pr
       const BN l2 = (hg::HostMont(pr2).pow2(pr - BN(1)) - BN(1)) / pr;
       const BN d = neg((l2 * BN(64)) % pr);
-      const BN lz = (R1h - inv2[sd]) % pr;
-      put2(o + (7 + sd) * H, neg((h * R1h) % pr), H);
-      put2(o + (9 + sd) * H, neg((d * h) % pr), H);
-      put2(o + (11 + sd) * H, neg((lz + d) % pr), H);
+      const BN lz = (R1h - BN::invmod(pr, R1h)) % pr;
+      put2((3 + sd) * H, neg((h * R1h) % pr), H);
+      put2((5 + sd) * H, neg((d * h) % pr), H);
+      put2((7 + sd) * H, neg((lz + d) % pr), H);
+      // digits of 2^(32 (H + 1)) mod pr^2
+      const BN rho = BN(1).shl(32 * ((size_t)H + 1)) % pr2;
+      put2(9 * H + sd * Sp, rho % pr, H);
+      put2(9 * H + sd * Sp + H, neg((rho / pr) % pr), H);
     }
     k->primes.assign(2 * (size_t)H, 0u);
     k->p.to_limbs(k->primes.data(), H);
@@ -1069,22 +1065,15 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
     cuda_check(cudaMemcpy(ds, hs2.data(), hs2.size() * 4, cudaMemcpyHostToDevice), "upload secret consts");
     auto& sc = k->sc;
     sc.Sp = Sp;
-    sc.P2[0] = ds;
-    sc.P2[1] = ds + Sp;
-    sc.P[0] = ds + o;
-    sc.P[1] = ds + o + H;
-    sc.hR[0] = ds + o + 2 * H;
-    sc.hR[1] = ds + o + 3 * H;
-    sc.inv2[0] = ds + o + 4 * H;
-    sc.inv2[1] = ds + o + 5 * H;
-    sc.pinvqR = ds + o + 6 * H;
+    sc.P[0] = ds;
+    sc.P[1] = ds + H;
+    sc.pinvqR = ds + 2 * H;
     for (int sd = 0; sd < 2; ++sd) {
-      sc.c1[sd] = ds + o + (7 + sd) * H;
-      sc.c2[sd] = ds + o + (9 + sd) * H;
-      sc.vz[sd] = ds + o + (11 + sd) * H;
+      sc.c1[sd] = ds + (3 + sd) * H;
+      sc.c2[sd] = ds + (5 + sd) * H;
+      sc.vz[sd] = ds + (7 + sd) * H;
+      sc.one[sd] = ds + 9 * H + sd * Sp;
     }
-    sc.np2[0] = neg_inv32(p2.d[0]);
-    sc.np2[1] = neg_inv32(q2.d[0]);
     sc.np1[0] = neg_inv32(k->p.d[0]);
     sc.np1[1] = neg_inv32(k->q.d[0]);
     // fewest products: (k/2) / (w + 1) windows and 2^(w-1) odd powers
@@ -1103,6 +1092,21 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
     }
     sc.prog[0] = dp;
     sc.prog[1] = dp + len;
+    {
+      // the batch kernel's windows, at the same places for both primes
+      constexpr int fw = hg::kBatchDecWindow;
+      const BN e[2] = {k->p - BN(1), k->q - BN(1)};
+      sc.fwin = (int)std::max<size_t>(1, (std::max(e[0].bitlen(), e[1].bitlen()) + fw - 1) / fw);
+      std::vector<uint8_t> fp(2 * (size_t)sc.fwin);
+      for (int sd = 0; sd < 2; ++sd)
+        for (int j = 0; j < sc.fwin; ++j)
+          for (int b = 0; b < fw; ++b)
+            if (e[sd].bit((size_t)(sc.fwin - 1 - j) * fw + b)) fp[(size_t)sd * sc.fwin + j] |= (uint8_t)(1u << b);
+      uint8_t* df = k->fprogs.ensure<uint8_t>(fp.size());
+      cuda_check(cudaMemcpy(df, fp.data(), fp.size(), cudaMemcpyHostToDevice), "upload prog");
+      sc.fprog[0] = df;
+      sc.fprog[1] = df + sc.fwin;
+    }
     sc.variant = 0;
   }
   std::lock_guard<std::mutex> lk(ctx->mu);
@@ -2409,15 +2413,24 @@ struct hg_batch {
 
 namespace {
 
-// Relative cost of one ciphertext of an op (Montgomery multiplications x S^2).
+// Relative cost of one ciphertext of an op: multiply-adds over S^2.
 double job_cost(const KeyRec& k, int op) {
   const double s2 = (double)k.S * k.S;
   switch (op) {
-    case hg::kBatchEncrypt: return (k.kc.npos + 2) * s2;
-    case hg::kBatchDecrypt: return 2.0 * (k.key_bits / 2 + k.key_bits / 12) * (s2 / 4);
-    case hg::kBatchMul: return 80.0 * s2;
-    default: return s2;
+    case hg::kBatchEncrypt: return (k.kc.npos + 7) * s2;  // 4 (S/2)^2 a product
+    case hg::kBatchDecrypt: return 2.0 * (k.key_bits / 2) * 1.35 * (s2 / 4);  // both sides, products of 4 (S/4)^2
+    case hg::kBatchMul: return 110.0 * s2;
+    default: return 2.0 * s2;
   }
+}
+
+// Scratch limbs of a warp that runs an op in variant set V.
+size_t job_warp_words(const KeyRec& k, int op, int V) {
+  if (op == hg::kBatchDecrypt && k.secret)
+    return ((size_t)1 << hg::kBatchDecWindow) * 32 * (size_t)(k.Sp / hg::tp_for(k.Sp, V));
+  if (op != hg::kBatchMul) return 1;
+  const size_t limbs = 32 * (size_t)(k.S / hg::tpi_for(k.S, V));
+  return (k.kc.two_digit ? (size_t)hg::mul_slots(k.wm) : (size_t)1 << (k.wm - 1)) * limbs;
 }
 
 // One job of a persistent batch, resolved against its key.
@@ -2461,21 +2474,12 @@ BatchPlan plan_batch(const std::vector<JobSpec>& specs, int V) {
     d.aux = J.aux;
     d.count = J.count;
     plan.jobs.push_back(d);
-    int per_pass;
-    if (J.op == hg::kBatchDecrypt) {
-      const int TP = hg::tp_for(k->Sp, V);
-      per_pass = 32 / (2 * TP);
-      plan.warp_words = std::max(plan.warp_words, (size_t)per_pass * 2 * ((size_t)1 << (k->sc.wd - 1)) * k->Sp);
-    } else {
-      const int TPI = hg::tpi_for(k->S, V);
-      per_pass = 32 / TPI;
-      if (J.op == hg::kBatchMul)
-        plan.warp_words = std::max(plan.warp_words, (size_t)per_pass * ((size_t)1 << (k->wm - 1)) * k->S);
-    }
-    // a throughput tile is four passes of a warp (fewer trips to the
-    // queue); a latency tile one pass, so a short batch spreads one chain
-    // per warp instead of queueing four chains behind each other on a warp
-    const size_t tile = (size_t)per_pass * (V == hg::kBatchLatencyVariant ? 1 : 4);
+    const int per_pass = J.op == hg::kBatchDecrypt ? 32 / (2 * hg::tp_for(k->Sp, V)) : 32 / hg::tpi_for(k->S, V);
+    plan.warp_words = std::max(plan.warp_words, job_warp_words(*k, J.op, V));
+    // an addition's tile is four passes of a warp (fewer trips to the queue),
+    // all others are one pass: a pass is hundreds of microseconds, and a short
+    // batch spreads one chain per warp instead of queueing four on a warp
+    const size_t tile = (size_t)per_pass * (V != hg::kBatchLatencyVariant && J.op == hg::kBatchAdd ? 4 : 1);
     const double c = job_cost(*k, J.op);
     for (size_t st = 0; st < J.count; st += tile) {
       const size_t cnt = std::min(tile, J.count - st);
@@ -2872,10 +2876,8 @@ int hg_server_create(hg_ctx* ctx, const hg_server_config* cfg, hg_server** out) 
       for (auto& kv : ctx->keys) {
         const KeyRec& k = *kv.second;
         if (k.scheme != 0) continue;  // the server serves ZPaillier keys only
-        warp_words = std::max(warp_words, (size_t)(32 / hg::tpi_for(k.S, c.variant)) * ((size_t)1 << (k.wm - 1)) * k.S);
-        if (k.secret)
-          warp_words = std::max(warp_words, (size_t)(32 / (2 * hg::tp_for(k.Sp, c.variant))) * 2 *
-                                                ((size_t)1 << (k.sc.wd - 1)) * k.Sp);
+        for (int V : {c.variant, hg::kBatchLatencyVariant})
+          for (int op : {hg::kBatchMul, hg::kBatchDecrypt}) warp_words = std::max(warp_words, job_warp_words(k, op, V));
       }
     }
     const size_t scratch = (size_t)hg::batch_resident_blocks(c.variant) * hg::batch_warps_per_block() * warp_words * 4;

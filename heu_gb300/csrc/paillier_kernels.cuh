@@ -54,25 +54,25 @@ struct KeyConst {
 
 // Secret-key constants for CRT decryption.  Index 0 = p side, 1 = q side.
 struct SecConst {
-  const uint32_t* P2[2];    // p^2, q^2                    (Sp limbs)
   const uint32_t* P[2];     // p, q                        (Sp/2 limbs)
-  const uint32_t* hR[2];    // hp*R1 mod p, hq*R1 mod q    (Sp/2 limbs), R1 = 2^(16*Sp)
-  const uint32_t* inv2[2];  // p^-1, q^-1 mod 2^(16*Sp)    (Sp/2 limbs)
-  const uint32_t* pinvqR;   // (p^-1 mod q)*R1 mod q       (Sp/2 limbs)
+  const uint32_t* pinvqR;   // (p^-1 mod q)*R1 mod q       (Sp/2 limbs), R1 = 2^(16*Sp)
   // two-digit decryption (decrypt_kernels.cu): with C^(p-1) = 1 + L p mod p^2,
   // delta = 2^-64 (what its input conversion leaves in C) and delta^(p-1) =
   // 1 + d p, digit 1 of the result is z = -(L + d): m_p = L hp = z*c1*R1^-1 + c2
   const uint32_t* c1[2];    // -hp*R1 mod p, -hq*R1 mod q  (Sp/2 limbs)
   const uint32_t* c2[2];    // -d*hp mod p, the same for q (Sp/2 limbs)
   const uint32_t* vz[2];    // z that stands for C = 0 mod p: L = -p^-1 mod R1
+  // the batch kernel's exponentiation (sq_decrypt.cuh)
+  const uint8_t* fprog[2];  // windows of p-1, q-1, highest first
+  const uint32_t* one[2];   // digits of 2^(16 Sp + 32) mod p^2, q^2 (Sp limbs)
+  int fwin;                 // windows of both
   const uint16_t* prog[2];  // exponent programs for p-1, q-1
-  uint32_t np2[2];          // -(p^2)^-1, -(q^2)^-1 mod 2^32
   uint32_t np1[2];          // -p^-1, -q^-1 mod 2^32
   int start[2];             // first window's table index
   int prog_len;             // both programs padded to this many steps
   int wd;                   // decryption window bits
   int Sp;                   // 32-bit limbs of p^2
-  int variant;              // (threads per unit side, limbs per thread) variant
+  int variant;              // 0, or 1: without the narrowest layout
 };
 
 // Okamoto-Uchiyama secret constants (ou/secret_key.h; decryptor.cc:27-45).
@@ -92,6 +92,8 @@ struct OuConst {
   int Sp;                 // 32-bit limbs of the p^2 arithmetic
 };
 
+// Window bits of the batch kernel's decryption (SecConst::fprog).
+constexpr int kBatchDecWindow = 5;
 // Table entries of a warp's scalar multiplication (sq_mul.cuh): the powers 0 ..
 // 2^wm - 1, then the constants into and out of the form of radix rho.
 __host__ __device__ constexpr int mul_slots(int wm) { return (1 << wm) + 2; }

@@ -1,6 +1,7 @@
-// Per-ciphertext operation bodies shared by the standalone kernels
-// (paillier_kernels.cu, decrypt_kernels.cu) and the persistent multi-key
-// batch kernel (batch_kernels.cu).
+// Per-ciphertext operation bodies modulo any n^2 (or an OU key's n), shared by
+// the standalone kernels (paillier_kernels.cu) and the persistent multi-key
+// batch kernel (batch_body.cuh).  ZPaillier keys encrypt, decrypt and multiply
+// in two digits instead (sq_*.cuh).
 //
 // Every *_one function processes one ciphertext per group of lanes: the
 // caller passes the clamped instance index `i` and whether it is `active`;
@@ -401,12 +402,7 @@ __device__ __forceinline__ void mul_bn_one(const KeyConst& kc, const uint32_t* _
   if (active) store_slice<L>(out + i * S + g.t * L, acc);
 }
 
-// ---------------------------------------------------------------------------
-// Decrypt (decryptor.cc:32-53): two groups per ciphertext, one per prime.
-//   x = REDC_p2(ct_mont) = c*Rp mod p^2;  y = x^(p-1) (sliding windows,
-//   shared exponent program);  y = REDC(y);  then one lane finishes
-//   L_p, CRT and the sign fold serially.
-// ---------------------------------------------------------------------------
+// One lane's serial Montgomery product (the tail of OU decryption).
 template <int H>
 __device__ __noinline__ void s_montmul(uint32_t* r, const uint32_t* a, const uint32_t* b, const uint32_t* m,
                                        uint32_t np) {
@@ -451,20 +447,6 @@ __device__ __noinline__ void s_montmul(uint32_t* r, const uint32_t* a, const uin
   for (int j = 0; j < H; ++j) r[j] = take ? d[j] : t[j];
 }
 
-template <int H>
-__device__ __forceinline__ uint32_t s_sub(uint32_t* r, const uint32_t* a, const uint32_t* b) {
-  int64_t br = 0;
-#pragma unroll 1
-  for (int j = 0; j < H; ++j) {
-    const int64_t v = (int64_t)a[j] - b[j] - br;
-    br = v < 0;
-    r[j] = (uint32_t)v;
-  }
-  return (uint32_t)br;
-}
-
-// Serial CRT tail for one ciphertext, run by one lane: y[0], y[1] = the
-// Z-form values c^(p-1) mod p^2 and c^(q-1) mod q^2 (SP = 2H limbs each).
 // Decoding of a decrypted plaintext (magnitude mm of W limbs, negative when
 // `neg`) under a device encoding, into out0 / cd.out1 (element i) and the
 // overflow flag:
@@ -552,196 +534,6 @@ __device__ void decode_plain(const Codec& cd, const uint32_t* mm, bool neg, size
   if (ovf) ovf[i] = neg ? 1 : 0;
 }
 
-template <int H>
-__device__ __noinline__ void crt_tail(const KeyConst& kc, const SecConst& sc, const uint32_t* y0,
-                                      const uint32_t* y1, size_t i, bool active, int64_t* __restrict__ out_i64,
-                                      uint8_t* __restrict__ out_ovf, uint32_t* __restrict__ out_mag,
-                                      uint8_t* __restrict__ out_neg, const Codec& cd) {
-  uint32_t Lv[H], mp[H], mq[H], t1[H];
-  // L_p = (y_p - 1)/p exactly = ((y_p - 1) mod 2^(32H)) * p^-1 mod 2^(32H)
-#pragma unroll 1
-  for (int sd = 0; sd < 2; ++sd) {
-    const uint32_t* y = sd == 0 ? y0 : y1;
-    uint64_t br = 1;
-#pragma unroll 1
-    for (int j = 0; j < H; ++j) {
-      const uint64_t v = (uint64_t)y[j] - br;
-      t1[j] = (uint32_t)v;
-      br = (v >> 63) & 1ull;
-    }
-    const uint32_t* iv = sc.inv2[sd];
-#pragma unroll 1
-    for (int j = 0; j < H; ++j) Lv[j] = 0;
-#pragma unroll 1
-    for (int a = 0; a < H; ++a) {
-      uint64_t c = 0;
-      const uint32_t ta = t1[a];
-#pragma unroll 1
-      for (int b = 0; a + b < H; ++b) {
-        c += (uint64_t)ta * iv[b] + Lv[a + b];
-        Lv[a + b] = (uint32_t)c;
-        c >>= 32;
-      }
-    }
-    s_montmul<H>(sd == 0 ? mp : mq, Lv, sc.hR[sd], sc.P[sd], sc.np1[sd]);
-  }
-  // mp mod q (p < 2q), d = mq - mp mod q, h = d * p^-1 mod q
-  const uint32_t* Q = sc.P[1];
-  uint32_t mpq[H];
-  {
-    const uint32_t b = s_sub<H>(t1, mp, Q);
-#pragma unroll 1
-    for (int j = 0; j < H; ++j) mpq[j] = b ? mp[j] : t1[j];
-  }
-  uint32_t dd[H];
-  {
-    const uint32_t b = s_sub<H>(dd, mq, mpq);
-    if (b) {
-      uint64_t c = 0;
-#pragma unroll 1
-      for (int j = 0; j < H; ++j) {
-        c += (uint64_t)dd[j] + Q[j];
-        dd[j] = (uint32_t)c;
-        c >>= 32;
-      }
-    }
-  }
-  uint32_t hh[H];
-  s_montmul<H>(hh, dd, sc.pinvqR, Q, sc.np1[1]);
-  // m = mp + p*h  (2H limbs)
-  uint32_t mm[2 * H];
-  const uint32_t* P = sc.P[0];
-#pragma unroll 1
-  for (int j = 0; j < 2 * H; ++j) mm[j] = j < H ? mp[j] : 0u;
-#pragma unroll 1
-  for (int a = 0; a < H; ++a) {
-    uint64_t c = 0;
-    const uint32_t pa = P[a];
-#pragma unroll 1
-    for (int b = 0; b < H; ++b) {
-      c += (uint64_t)pa * hh[b] + mm[a + b];
-      mm[a + b] = (uint32_t)c;
-      c >>= 32;
-    }
-#pragma unroll 1
-    for (int j = a + H; c && j < 2 * H; ++j) {
-      c += mm[j];
-      mm[j] = (uint32_t)c;
-      c >>= 32;
-    }
-  }
-  // sign fold: m > n/2 => m - n (decryptor.cc:49-52)
-  bool gt = false;
-#pragma unroll 1
-  for (int j = 2 * H - 1; j >= 0; --j) {
-    const uint32_t hv = kc.nhalf[j];
-    if (mm[j] != hv) {
-      gt = mm[j] > hv;
-      break;
-    }
-  }
-  if (gt) {
-    int64_t br = 0;
-#pragma unroll 1
-    for (int j = 0; j < 2 * H; ++j) {
-      const int64_t v = (int64_t)kc.n[j] - mm[j] - br;
-      br = v < 0;
-      mm[j] = (uint32_t)v;
-    }
-  }
-  if (active && cd.kind != kCodecNone) {
-    decode_plain<2 * H>(cd, mm, gt, i, out_i64, out_ovf);
-    return;
-  }
-  if (active) {
-    if (out_mag) {
-#pragma unroll 1
-      for (int j = 0; j < 2 * H; ++j) out_mag[i * (2 * H) + j] = mm[j];
-      out_neg[i] = gt ? 1 : 0;
-    }
-    if (out_i64) {
-      bool fits = true;
-#pragma unroll 1
-      for (int j = 2; j < 2 * H; ++j) fits &= (mm[j] == 0u);
-      const uint64_t mag = (uint64_t)mm[0] | ((uint64_t)mm[1] << 32);
-      if (gt) {
-        fits &= mag <= (1ull << 63);
-        out_i64[i] = (int64_t)((uint64_t)0 - mag);
-      } else {
-        fits &= mag < (1ull << 63);
-        out_i64[i] = (int64_t)mag;
-      }
-      if (out_ovf) out_ovf[i] = fits ? 0 : 1;
-    }
-  }
-}
-
-// One ciphertext per pair of groups: `side` 0 works mod p^2, 1 mod q^2.
-// `tb` is this group's odd-power table (offset by the lane's slice), `ysm`
-// this ciphertext's hand-off buffer of 2 x SP limbs in shared memory.
-template <int TP, int LP>
-__device__ __forceinline__ void decrypt_one(const KeyConst& kc, const SecConst& sc, const uint32_t* __restrict__ ct,
-                                            size_t i, bool active, int side, uint32_t* __restrict__ tb,
-                                            uint32_t* ysm, int64_t* __restrict__ out_i64,
-                                            uint8_t* __restrict__ out_ovf, uint32_t* __restrict__ out_mag,
-                                            uint8_t* __restrict__ out_neg, const Group<TP>& g, uint32_t* err,
-                                            const Codec& cd = Codec{}) {
-  constexpr int SP = TP * LP;
-  const int ntab = 1 << (sc.wd - 1);
-  uint32_t N[LP];
-  load_slice<LP>(N, sc.P2[side] + g.t * LP);
-  const uint32_t np = sc.np2[side];
-  const uint16_t* prog = sc.prog[side];
-  uint32_t lo[LP], hi[LP], x[LP];
-  load_slice<LP>(lo, ct + i * (2 * SP) + g.t * LP);
-  load_slice<LP>(hi, ct + i * (2 * SP) + SP + g.t * LP);
-  {
-    // validate against n^2 (decryptor.cc:21-23)
-    uint32_t Nlo[LP], Nhi[LP], d[LP];
-    load_slice<LP>(Nlo, kc.N + g.t * LP);
-    load_slice<LP>(Nhi, kc.N + SP + g.t * LP);
-    const uint32_t b_lo = sub_full<TP, LP>(d, lo, Nlo, g);
-    uint32_t e2[LP];
-    (void)sub_full<TP, LP>(e2, hi, Nhi, g);
-    const bool hi_lt = less_than<TP, LP>(hi, Nhi, g);
-    const bool hi_eq = is_zero<TP, LP>(e2, g);
-    const bool ok = hi_lt || (hi_eq && b_lo);
-    if (active && !ok && g.t == 0 && side == 0) atomicOr(err, kErrCtRange);
-  }
-  mont_redc_wide<TP, LP>(x, lo, hi, N, np, g);
-  store_slice<LP>(tb, x);
-  uint32_t x2[LP], cur[LP];
-  mont_mul<TP, LP>(x2, x, x, N, np, g);
-  copy_slice<LP>(cur, x);
-#pragma unroll 1
-  for (int t = 1; t < ntab; ++t) {
-    mont_mul<TP, LP>(cur, cur, x2, N, np, g);
-    store_slice<LP>(tb + (size_t)t * SP, cur);
-  }
-  uint32_t acc[LP];
-  load_slice<LP>(acc, tb + (size_t)sc.start[side] * SP);
-#pragma unroll 1
-  for (int s = 0; s < sc.prog_len; ++s) {
-    const uint16_t op = prog[s];
-    uint32_t B[LP];
-    if (op < kOpNop) {
-      load_slice<LP>(B, tb + (size_t)op * SP);
-    } else {
-      copy_slice<LP>(B, acc);
-    }
-    uint32_t res[LP];
-    mont_mul<TP, LP>(res, acc, B, N, np, g);
-    if (op != kOpNop) copy_slice<LP>(acc, res);
-  }
-  mont_redc<TP, LP>(acc, acc, N, np, g);
-#pragma unroll
-  for (int j = 0; j < LP; ++j) ysm[side * SP + g.t * LP + j] = acc[j];
-  __syncwarp();
-  if (side == 0 && g.t == 0)
-    crt_tail<SP / 2>(kc, sc, ysm, ysm + SP, i, active, out_i64, out_ovf, out_mag, out_neg, cd);
-  __syncwarp();
-}
-
 // Montgomery conversion: to_mont = MM(x, R^2), from_mont = REDC(x)
 template <int TPI, int L>
 __device__ __forceinline__ void convert_one(const KeyConst& kc, const uint32_t* __restrict__ in,
@@ -797,32 +589,13 @@ __device__ __forceinline__ size_t next_work(unsigned long long* ctr, int per_war
     default: return cudaErrorInvalidValue;                                               \
   }
 
-#define HG_DISPATCH_SPV(SP, V, ...)                                                      \
-  switch ((SP) * 2 + ((V) ? 1 : 0)) {                                                    \
-    case 64: { constexpr int TP = 2, LP = 16; __VA_ARGS__; } break;                      \
-    case 65: { constexpr int TP = 4, LP = 8; __VA_ARGS__; } break;                       \
-    case 128: { constexpr int TP = 4, LP = 16; __VA_ARGS__; } break;                     \
-    case 129: { constexpr int TP = 8, LP = 8; __VA_ARGS__; } break;                      \
-    case 192: { constexpr int TP = 8, LP = 12; __VA_ARGS__; } break;                     \
-    case 193: { constexpr int TP = 4, LP = 24; __VA_ARGS__; } break;                     \
-    default: return cudaErrorInvalidValue;                                               \
-  }
-
-// Latency layout (short batches): a whole warp per instance mod n^2 and a
-// half warp per CRT side mod p^2, so each dependent chain of Montgomery
-// multiplications advances with 2-6 limbs per lane instead of 8-24.
+// Latency layout (short batches): a whole warp per instance mod n^2, so each
+// dependent chain of Montgomery multiplications advances with 2-6 limbs per
+// lane instead of 8-24.
 #define HG_DISPATCH_SL(S, ...)                                                           \
   switch (S) {                                                                           \
     case 64: { constexpr int TPI = 32, L = 2; __VA_ARGS__; } break;                      \
     case 128: { constexpr int TPI = 32, L = 4; __VA_ARGS__; } break;                     \
     case 192: { constexpr int TPI = 32, L = 6; __VA_ARGS__; } break;                     \
-    default: return cudaErrorInvalidValue;                                               \
-  }
-
-#define HG_DISPATCH_SPL(SP, ...)                                                         \
-  switch (SP) {                                                                          \
-    case 32: { constexpr int TP = 16, LP = 2; __VA_ARGS__; } break;                      \
-    case 64: { constexpr int TP = 16, LP = 4; __VA_ARGS__; } break;                      \
-    case 96: { constexpr int TP = 16, LP = 6; __VA_ARGS__; } break;                      \
     default: return cudaErrorInvalidValue;                                               \
   }

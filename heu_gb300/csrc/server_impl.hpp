@@ -107,8 +107,8 @@ size_t slice_dev_bytes(const KeyRec& k, const hg_request& r, size_t n) {
 // Estimated GPU time of one element of an op, in microseconds (cost model
 // used to size micro-batches; the kernels do not depend on it).
 double elem_cost_us(const KeyRec& k, int op) {
-  if (op == kOpSum) return (double)k.S * k.S / 3.11e6;
-  return job_cost(k, op) / 3.11e6;
+  if (op == kOpSum) return 2.0 * (double)k.S * k.S / 8.8e6;
+  return job_cost(k, op) / 8.3e6;
 }
 
 }  // namespace
