@@ -103,14 +103,13 @@ __device__ __forceinline__ void sq_stage(uint32_t* area, const uint32_t (&x)[L],
 
 // Reduction of one limb in both chains, then the shift by one limb.  The
 // pending c1 must be 0.  `in` enters the top limb of chain 0.  Without kJoin
-// the chains are two reductions modulo n of their own.
-template <int TC, int L, bool kJoin = true, class Mod>
-__device__ __forceinline__ void sq_reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t& ov, uint32_t& c1,
-                                               const Mod& n, uint32_t np, uint32_t in, const SqLanes<TC, L>& g) {
-  // both chains' lowest limbs travel together, so that chain 1 finds its m
-  // (which depends on chain 0's) after one shuffle instead of two
-  const uint32_t a = __shfl_sync(kFull, Ev[0], g.base);
-  const uint32_t b = TC > 1 ? __shfl_sync(kFull, Ev[0], g.base + TC) : Ev[0];
+// the chains are two reductions modulo n of their own.  a, b: the lowest limbs
+// of the instance's chains, which travel together so that chain 1 finds its m
+// (it depends on chain 0's) after one shuffle's time and not two.
+template <int TC, int L, bool kJoin, class Mod>
+__device__ __forceinline__ void sq_reduce_with(uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t& ov, uint32_t& c1,
+                                               const Mod& n, uint32_t np, uint32_t in, uint32_t a, uint32_t b,
+                                               const SqLanes<TC, L>& g) {
   const uint32_t m0 = a * np;
   const uint32_t m = g.c ? (kJoin ? b + m0 : b) * np : m0;
   row_mac<L>(Ev, Od, ov, (kJoin && g.c == 1 && g.t == 0) ? m0 : 0u, n, m);
@@ -123,6 +122,32 @@ __device__ __forceinline__ void sq_reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)
   Ev[L - 2] = w;
   Ev[L - 1] = ov;
   ov = 0u;
+}
+
+template <int TC, int L, bool kJoin = true, class Mod>
+__device__ __forceinline__ void sq_reduce_step(uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t& ov, uint32_t& c1,
+                                               const Mod& n, uint32_t np, uint32_t in, const SqLanes<TC, L>& g) {
+  const uint32_t a = __shfl_sync(kFull, Ev[0], g.base);
+  const uint32_t b = TC > 1 ? __shfl_sync(kFull, Ev[0], g.base + TC) : Ev[0];
+  sq_reduce_with<TC, L, kJoin>(Ev, Od, ov, c1, n, np, in, a, b, g);
+}
+
+// One step of the layouts for few ciphertexts, where the chain of dependent
+// instructions sets the time: `low` is this step's lowest limb in the chains'
+// first lanes, found ahead of the rows, so its shuffle runs under the product
+// rows; the next step's is Od[0] + Ev[1] after the reduction row plus `next`,
+// the lowest limb of its products.
+template <int TC, int L, bool kTwo, bool kJoin, class Mod>
+__device__ __forceinline__ void sq_step_early(uint32_t (&Ev)[L], uint32_t (&Od)[L], uint32_t& ov, uint32_t& c1,
+                                              uint32_t& low, uint32_t next, const uint32_t (&x)[L], uint32_t y,
+                                              const uint32_t (&x2)[L], uint32_t y2, const Mod& n, uint32_t np,
+                                              const SqLanes<TC, L>& g) {
+  const uint32_t a = __shfl_sync(kFull, low, g.base);
+  const uint32_t b = __shfl_sync(kFull, low, g.base + TC);
+  row_mac<L>(Ev, Od, ov, c1, x, y);
+  if constexpr (kTwo) row_mac<L>(Ev, Od, ov, 0u, x2, y2);
+  sq_reduce_with<TC, L, kJoin>(Ev, Od, ov, c1, n, np, 0u, a, b, g);
+  low = Od[0] + c1 + next;
 }
 
 // Columns -> limbs of both chains' results, below 2^(32 H).
@@ -177,6 +202,15 @@ __device__ __forceinline__ void sq_settle(uint32_t (&x)[L], const uint32_t (&Ev)
 template <int TC, int L>
 constexpr int kSqUnroll = TC == 1 && L == 32 ? 8 : 16;
 
+// Layouts whose passes run sq_step_early: the widest of the primes' lengths,
+// which only few ciphertexts take.  8 CRT decryptions of 2048 bits (16 lanes a
+// chain) took 1.92 ms without and 1.71 with it, 3072 bits (8 lanes) 5.20 and
+// 4.90.  With 4 limbs a lane and more steps a pass it gains nothing (one
+// encryption of 2048 bits 0.102 and 0.104 ms), and with several warps a
+// scheduler its extra work costs 2 to 3%.
+template <int TC, int L>
+constexpr bool kSqEarly = L == 2 || (TC == 8 && L == 6);
+
 // z = (x * y [+ x2 * y2]) / rho in both chains, chain 0's m entering chain 1.
 // y: this lane's multiplier limbs in shared memory (limb 0), doubled when
 // `dbl` is 1.  kTwo adds the second product row.  z may alias x.
@@ -196,30 +230,61 @@ __device__ __forceinline__ void sq_pass(uint32_t (&z)[L], const uint32_t (&x)[L]
 #pragma unroll
   for (int j = 0; j < L; ++j) E[j] = O[j] = 0u;
   uint32_t ov = 0u, c1 = 0u, prev = 0u;
-#pragma unroll 1
-  for (int i = 0; i < H; i += kU) {
-#pragma unroll
-    for (int k = 0; k < kU; k += 4) {
-      const uint4 q = *reinterpret_cast<const uint4*>(y + (i + k) * IPW);
-      const uint4 q2 = kTwo ? *reinterpret_cast<const uint4*>(y2 + (i + k) * IPW) : make_uint4(0u, 0u, 0u, 0u);
-      row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, q.x, dbl));
-      if constexpr (kTwo) row_mac<L>(E, O, ov, 0u, x2, g.c ? q2.x : 0u);
-      sq_reduce_step<TC, L, kJoin>(E, O, ov, c1, n, np, 0u, g);
-      row_mac<L>(O, E, ov, c1, x, __funnelshift_l(q.x, q.y, dbl));
-      if constexpr (kTwo) row_mac<L>(O, E, ov, 0u, x2, g.c ? q2.y : 0u);
-      sq_reduce_step<TC, L, kJoin>(O, E, ov, c1, n, np, 0u, g);
-      row_mac<L>(E, O, ov, c1, x, __funnelshift_l(q.y, q.z, dbl));
-      if constexpr (kTwo) row_mac<L>(E, O, ov, 0u, x2, g.c ? q2.z : 0u);
-      sq_reduce_step<TC, L, kJoin>(E, O, ov, c1, n, np, 0u, g);
-      row_mac<L>(O, E, ov, c1, x, __funnelshift_l(q.z, q.w, dbl));
-      if constexpr (kTwo) row_mac<L>(O, E, ov, 0u, x2, g.c ? q2.w : 0u);
-      sq_reduce_step<TC, L, kJoin>(O, E, ov, c1, n, np, 0u, g);
-      prev = q.w;
+  if constexpr ((kSqEarly<TC, L>)) {
+    uint4 q = *reinterpret_cast<const uint4*>(y);
+    uint4 q2 = kTwo ? *reinterpret_cast<const uint4*>(y2) : make_uint4(0u, 0u, 0u, 0u);
+    if (kTwo && !g.c) q2 = make_uint4(0u, 0u, 0u, 0u);
+    // the lowest limb of the products of multiplier limbs v (and w)
+    auto lowest = [&](uint32_t v, uint32_t w) { return kTwo ? x[0] * v + x2[0] * w : x[0] * v; };
+    uint32_t v0 = __funnelshift_l(0u, q.x, dbl);
+    uint32_t low = lowest(v0, q2.x);
+#pragma unroll 4
+    for (int i = 0; i < H; i += 4) {
+      const int at = i + 4 < H ? (i + 4) * IPW : 0;
+      uint4 p = *reinterpret_cast<const uint4*>(y + at);
+      uint4 p2 = kTwo ? *reinterpret_cast<const uint4*>(y2 + at) : make_uint4(0u, 0u, 0u, 0u);
+      if (kTwo && !g.c) p2 = make_uint4(0u, 0u, 0u, 0u);
+      if (i + 4 >= H) {
+        p.x = ytop;
+        p2.x = 0u;
+      }
+      const uint32_t v1 = __funnelshift_l(q.x, q.y, dbl), v2 = __funnelshift_l(q.y, q.z, dbl);
+      const uint32_t v3 = __funnelshift_l(q.z, q.w, dbl), v4 = __funnelshift_l(q.w, p.x, dbl);
+      sq_step_early<TC, L, kTwo, kJoin>(E, O, ov, c1, low, lowest(v1, q2.y), x, v0, x2, q2.x, n, np, g);
+      sq_step_early<TC, L, kTwo, kJoin>(O, E, ov, c1, low, lowest(v2, q2.z), x, v1, x2, q2.y, n, np, g);
+      sq_step_early<TC, L, kTwo, kJoin>(E, O, ov, c1, low, lowest(v3, q2.w), x, v2, x2, q2.z, n, np, g);
+      sq_step_early<TC, L, kTwo, kJoin>(O, E, ov, c1, low, lowest(v4, p2.x), x, v3, x2, q2.w, n, np, g);
+      v0 = v4;
+      q = p;
+      q2 = p2;
     }
+    sq_step_early<TC, L, false, kJoin>(E, O, ov, c1, low, 0u, x, v0, x2, 0u, n, np, g);
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < H; i += kU) {
+#pragma unroll
+      for (int k = 0; k < kU; k += 4) {
+        const uint4 q = *reinterpret_cast<const uint4*>(y + (i + k) * IPW);
+        const uint4 q2 = kTwo ? *reinterpret_cast<const uint4*>(y2 + (i + k) * IPW) : make_uint4(0u, 0u, 0u, 0u);
+        row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, q.x, dbl));
+        if constexpr (kTwo) row_mac<L>(E, O, ov, 0u, x2, g.c ? q2.x : 0u);
+        sq_reduce_step<TC, L, kJoin>(E, O, ov, c1, n, np, 0u, g);
+        row_mac<L>(O, E, ov, c1, x, __funnelshift_l(q.x, q.y, dbl));
+        if constexpr (kTwo) row_mac<L>(O, E, ov, 0u, x2, g.c ? q2.y : 0u);
+        sq_reduce_step<TC, L, kJoin>(O, E, ov, c1, n, np, 0u, g);
+        row_mac<L>(E, O, ov, c1, x, __funnelshift_l(q.y, q.z, dbl));
+        if constexpr (kTwo) row_mac<L>(E, O, ov, 0u, x2, g.c ? q2.z : 0u);
+        sq_reduce_step<TC, L, kJoin>(E, O, ov, c1, n, np, 0u, g);
+        row_mac<L>(O, E, ov, c1, x, __funnelshift_l(q.z, q.w, dbl));
+        if constexpr (kTwo) row_mac<L>(O, E, ov, 0u, x2, g.c ? q2.w : 0u);
+        sq_reduce_step<TC, L, kJoin>(O, E, ov, c1, n, np, 0u, g);
+        prev = q.w;
+      }
+    }
+    // the extra limb of rho: a doubled multiplier's top bit, or ytop
+    row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, ytop, dbl));
+    sq_reduce_step<TC, L, kJoin>(E, O, ov, c1, n, np, 0u, g);
   }
-  // the extra limb of rho: a doubled multiplier's top bit, or ytop
-  row_mac<L>(E, O, ov, c1, x, __funnelshift_l(prev, ytop, dbl));
-  sq_reduce_step<TC, L, kJoin>(E, O, ov, c1, n, np, 0u, g);
   sq_settle<TC, L, kJoin>(z, O, E, c1, n, g);
 }
 
