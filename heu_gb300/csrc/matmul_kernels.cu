@@ -234,8 +234,29 @@ cudaError_t launch_row_products(int S, const KeyConst& kc, const uint32_t* T, si
   return cudaGetLastError();
 }
 
+// Rows up to which a power runs with a warp per row: one wave at 12 per SM.
+// Its time there is that of one row's chain of products, shorter with fewer
+// limbs a lane, as for the inverse tree's small levels (paillier_kernels.cu).
+static bool few_rows(size_t count) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return count <= (size_t)12 * std::max(sms, 1);
+}
+#define HG_DISPATCH_S3L(S, ...)                                         \
+  switch (S) {                                                          \
+    case 64: { constexpr int TPI = 32, L = 2; __VA_ARGS__; } break;     \
+    case 128: { constexpr int TPI = 32, L = 4; __VA_ARGS__; } break;    \
+    case 192: { constexpr int TPI = 32, L = 6; __VA_ARGS__; } break;    \
+    default: return cudaErrorInvalidValue;                              \
+  }
+
 cudaError_t launch_pow_shared(int S, const KeyConst& kc, uint32_t* v, size_t count, uint64_t e, cudaStream_t st) {
   if (e <= 1) return cudaSuccess;
+  if (few_rows(count)) {
+    HG_DISPATCH_S3L(S, k_pow_shared<TPI, L><<<nblocks(count, TPI), kBlock, 0, st>>>(kc, v, count, e));
+    return cudaGetLastError();
+  }
   HG_DISPATCH_S3(S, k_pow_shared<TPI, L><<<nblocks(count, TPI), kBlock, 0, st>>>(kc, v, count, e));
   return cudaGetLastError();
 }
@@ -243,6 +264,10 @@ cudaError_t launch_pow_shared(int S, const KeyConst& kc, uint32_t* v, size_t cou
 cudaError_t launch_pow_shared_bn(int S, const KeyConst& kc, uint32_t* v, size_t count, const uint32_t* e, int el,
                                  cudaStream_t st) {
   if (count == 0 || el < 1) return cudaSuccess;
+  if (few_rows(count)) {
+    HG_DISPATCH_S3L(S, k_pow_shared_bn<TPI, L><<<nblocks(count, TPI), kBlock, 0, st>>>(kc, v, count, e, el));
+    return cudaGetLastError();
+  }
   HG_DISPATCH_S3(S, k_pow_shared_bn<TPI, L><<<nblocks(count, TPI), kBlock, 0, st>>>(kc, v, count, e, el));
   return cudaGetLastError();
 }
