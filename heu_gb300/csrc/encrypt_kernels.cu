@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(64) k_sq_bases(const __grid_constant__ KeyCons
 template <int TC, int L>
 __global__ void __launch_bounds__(128) k_sq_level(const __grid_constant__ KeyConst kc, uint32_t* __restrict__ table,
                                                   uint32_t* __restrict__ inv, const uint32_t* __restrict__ bases,
-                                                  int pos0, int npos, int level) {
+                                                  int pos0, size_t npos, int level, int subset) {
   using G = SqLanes<TC, L>;
   constexpr int H = G::H, S = 2 * H;
   __shared__ __align__(16) uint32_t areas[4][4 * G::kDigit];
@@ -127,9 +127,9 @@ __global__ void __launch_bounds__(128) k_sq_level(const __grid_constant__ KeyCon
   const size_t ent = (size_t)((1u << kc.w) - 1u);
   const bool scale = level == kc.w;
   const size_t lo = level < 0 || scale ? 1 : (1ull << level) + 1ull;
-  const size_t hi = level < 0 ? 1 : scale ? ent : min((size_t)(1ull << (level + 1)), ent);
+  const size_t hi = level < 0 ? 1 : scale ? ent : min((size_t)(1ull << (level + 1)) - (subset ? 1 : 0), ent);
   if (hi < lo) return;
-  const size_t per = hi - lo + 1, total = per * (size_t)npos;
+  const size_t per = hi - lo + 1, total = per * npos;
   const size_t pair = ((size_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * G::IPW;
   if (2 * pair >= total) return;
   // this group's two entries; past the end the last one again
@@ -279,18 +279,18 @@ cudaError_t launch_sq_bases(int S, const KeyConst& kc, const uint32_t* first, ui
 }
 
 cudaError_t launch_sq_level(int S, const KeyConst& kc, uint32_t* table, uint32_t* inv, const uint32_t* bases, int pos0,
-                            int npos, int level, cudaStream_t st) {
+                            size_t npos, int level, int subset, cudaStream_t st) {
   const size_t ent = (size_t)((1u << kc.w) - 1u);
   const bool scale = level == kc.w;
   const size_t lo = level < 0 || scale ? 1 : ((size_t)1 << level) + 1;
-  const size_t hi = level < 0 ? 1 : scale ? ent : std::min((size_t)1 << (level + 1), ent);
+  const size_t hi = level < 0 ? 1 : scale ? ent : std::min(((size_t)1 << (level + 1)) - (subset ? 1 : 0), ent);
   if (hi < lo) return cudaSuccess;
-  const size_t pairs = ((hi - lo + 1) * (size_t)npos + 1) / 2;
+  const size_t pairs = ((hi - lo + 1) * npos + 1) / 2;
   // 16 limbs a lane (12 at 3072 bits): enough groups for the small levels
   switch (S) {
-    case 64: k_sq_level<2, 16><<<(unsigned)((pairs + 31) / 32), 128, 0, st>>>(kc, table, inv, bases, pos0, npos, level); break;
-    case 128: k_sq_level<4, 16><<<(unsigned)((pairs + 15) / 16), 128, 0, st>>>(kc, table, inv, bases, pos0, npos, level); break;
-    case 192: k_sq_level<8, 12><<<(unsigned)((pairs + 7) / 8), 128, 0, st>>>(kc, table, inv, bases, pos0, npos, level); break;
+    case 64: k_sq_level<2, 16><<<(unsigned)((pairs + 31) / 32), 128, 0, st>>>(kc, table, inv, bases, pos0, npos, level, subset); break;
+    case 128: k_sq_level<4, 16><<<(unsigned)((pairs + 15) / 16), 128, 0, st>>>(kc, table, inv, bases, pos0, npos, level, subset); break;
+    case 192: k_sq_level<8, 12><<<(unsigned)((pairs + 7) / 8), 128, 0, st>>>(kc, table, inv, bases, pos0, npos, level, subset); break;
     default: return cudaErrorInvalidValue;
   }
   count_launches(1);

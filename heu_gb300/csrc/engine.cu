@@ -258,7 +258,7 @@ struct Work {
   DevBuf scratch, red[2];
   TreeBufs inv;
   DevBuf seg_cnt, seg_offs[3], seg_cursor, seg_idx, seg_nch, seg_part[2];
-  DevBuf mm_tables, mm_masks, mm_prod, mm_exp;
+  DevBuf mm_tables, mm_masks, mm_prod, mm_exp, mm_inv, mm_tree;
   DevBuf sel;  // signs of multi-limb scalars as the inverse's selector
   DevBuf ou_e[2];
   DevBuf err;
@@ -773,6 +773,90 @@ void core_bucket_sum(KeyRec& k, Work& w, const uint32_t* x, size_t rows, size_t 
   }
 }
 
+// Bit planes of y' as lookup masks: masks[(j * P + plane) * nch + c] = bits of
+// y'(b c .. b c + b - 1, j) in `plane`.
+template <typename Bit>
+std::vector<uint8_t> plane_masks(size_t K, size_t N, int P, int b, Bit&& bit) {
+  const size_t nch = (K + b - 1) / b;
+  std::vector<uint8_t> hm(N * P * nch, 0);
+  for (size_t j = 0; j < N; ++j)
+    for (int plane = 0; plane < P; ++plane)
+      for (size_t kk = 0; kk < K; ++kk)
+        if (bit(kk, j, plane)) hm[(j * P + plane) * nch + kk / b] |= (uint8_t)(1u << (kk % b));
+  return hm;
+}
+
+// prod[i]^-o into the rows of out: one inverse and one power per row.
+void scale_by_offset(KeyRec& k, Work& w, uint32_t* prod, size_t r0, size_t rows, size_t N, const BN& o,
+                     const uint32_t* dexp, size_t exp_limbs, uint32_t* out) {
+  core_inverse(k, w, prod, nullptr, prod, rows);
+  if (dexp)
+    cuda_check(hg::launch_pow_shared_bn(k.S, k.kc, prod, rows, dexp, (int)exp_limbs, w.stream), "row power");
+  else
+    cuda_check(hg::launch_pow_shared(k.S, k.kc, prod, rows, o.low64(), w.stream), "row power");
+  cuda_check(hg::launch_scale_rows(k.S, k.kc, out, prod, r0, rows, (int)N, w.stream), "scale rows");
+}
+
+// MatMul in two digits (sq_matmul.cu); false where a base shares a factor
+// with n, which the kernels modulo n^2 then serve.
+template <typename Bit>
+bool matmul_two_digit(KeyRec& k, Work& w, const uint32_t* x, size_t M, size_t K, size_t N, int P, Bit&& bit,
+                      const BN& o, const uint32_t* dexp, size_t exp_limbs, uint32_t* out) {
+  const int b = hg::sq_matmul_chunk(K, N, (size_t)P);
+  const size_t S = (size_t)k.S, H = S / 2, nch = (K + b - 1) / b, ent = ((size_t)1 << b) - 1;
+  std::vector<uint8_t> hm = plane_masks(K, N, P, b, bit);
+  const size_t row_masks = hm.size();  // then the full masks of the row products
+  hm.insert(hm.end(), nch, (uint8_t)ent);
+  uint8_t* dmask = w.mm_masks.ensure<uint8_t>(hm.size());
+  cuda_check(cudaMemcpyAsync(dmask, hm.data(), hm.size(), cudaMemcpyHostToDevice, w.stream), "H2D masks");
+  const size_t per_row = nch * ent * (S + H) * 4;
+  const size_t Rb = std::max<size_t>(1, std::min(M, ((size_t)8 << 30) / per_row));
+  uint32_t* T = w.mm_tables.ensure<uint32_t>(Rb * nch * ent * S * 4);
+  uint32_t* inv = w.mm_inv.ensure<uint32_t>(Rb * nch * ent * H * 4);
+  uint32_t* tree = w.mm_tree.ensure<uint32_t>(tree_nodes(Rb * nch * b) * H * 4);
+  uint32_t* prod = w.mm_prod.ensure<uint32_t>(Rb * S * 4);
+  uint32_t* root = w.pin_root.ensure<uint32_t>(S * 4 + 4);
+  hg::KeyConst kt = k.kc;  // the tables' level kernel counts levels in w
+  kt.w = b;
+  bool units = true;
+  for (size_t r0 = 0; r0 < M && units; r0 += Rb) {
+    const size_t rows = std::min(Rb, M - r0);
+    cuda_check(hg::launch_mm_bases(k.S, k.kc, x, r0, rows, (int)K, b, T, tree, w.errp(), w.stream), "matmul bases");
+    std::vector<size_t> off{0}, size{rows * nch * b};
+    while (size.back() > 1) {
+      off.push_back(off.back() + size.back());
+      size.push_back((size.back() + 1) / 2);
+      const size_t l = size.size() - 1;
+      cuda_check(hg::launch_half_up(k.S, k.kc, tree + off[l - 1] * H, size[l - 1], tree + off[l] * H, w.stream),
+                 "matmul tree");
+    }
+    cuda_check(cudaMemcpyAsync(root, tree + off.back() * H, H * 4, cudaMemcpyDeviceToHost, w.stream), "D2H root");
+    cuda_check(cudaStreamSynchronize(w.stream), "stream sync");
+    // rho^2 / root = (2^(64 H) / root) 2^64
+    const std::vector<uint32_t> v = (BN::from_limbs(root, H) % k.n).limbs(H);
+    std::vector<uint32_t> z(H);
+    units = hg::mont_root_inverse(v.data(), k.n, H, z.data());
+    if (!units) break;
+    ((BN::from_limbs(z.data(), H) * BN(1).shl(64)) % k.n).to_limbs(root, H);
+    cuda_check(cudaMemcpyAsync(tree + off.back() * H, root, H * 4, cudaMemcpyHostToDevice, w.stream), "H2D inverse");
+    for (size_t l = size.size() - 1; l-- > 0;)
+      cuda_check(hg::launch_half_down(k.S, k.kc, tree + off[l] * H, size[l], tree + off[l + 1] * H, w.stream),
+                 "matmul tree");
+    cuda_check(hg::launch_mm_log(k.S, k.kc, rows, (int)K, b, T, tree, inv, w.stream), "matmul bases");
+    for (int lv = 1; lv < b; ++lv)
+      cuda_check(hg::launch_sq_level(k.S, kt, T, inv, nullptr, 0, rows * nch, lv, 1, w.stream), "matmul tables");
+    cuda_check(hg::launch_mm_planes(k.S, k.kc, T, dmask, r0, rows, (int)N, P, (int)K, b, out, w.stream),
+               "matmul planes");
+    if (!o.is_zero()) {
+      cuda_check(hg::launch_mm_planes(k.S, k.kc, T, dmask + row_masks, 0, rows, 1, 1, (int)K, b, prod, w.stream),
+                 "row products");
+      scale_by_offset(k, w, prod, r0, rows, N, o, dexp, exp_limbs, out);
+    }
+  }
+  cuda_check(cudaStreamSynchronize(w.stream), "stream sync");  // the masks' copy has run
+  return units;
+}
+
 // numpy MatMul of ciphertexts x (M x K) by int64 plaintexts y (K x N, host).
 // MatMul over exponents given as bit planes: bit(kk, j, plane) is bit `plane`
 // of y'(kk, j) = y(kk, j) + o >= 0 (P planes); o >= 0 is undone per row with
@@ -780,20 +864,6 @@ void core_bucket_sum(KeyRec& k, Work& w, const uint32_t* x, size_t rows, size_t 
 template <typename Bit>
 void core_matmul_planes(KeyRec& k, Work& w, const uint32_t* x, size_t M, size_t K, size_t N, int P, Bit&& bit,
                         const BN& o, uint32_t* out) {
-  const int nch = (int)((K + 7) / 8);
-  std::vector<uint8_t> hm((size_t)N * P * nch, 0);
-  for (size_t j = 0; j < N; ++j)
-    for (int plane = 0; plane < P; ++plane)
-      for (int c = 0; c < nch; ++c) {
-        uint8_t mk = 0;
-        for (int b = 0; b < 8; ++b) {
-          const size_t kk = (size_t)c * 8 + b;
-          if (kk < K && bit(kk, j, plane)) mk |= (uint8_t)(1u << b);
-        }
-        hm[((size_t)j * P + plane) * nch + c] = mk;
-      }
-  uint8_t* dmask = w.mm_masks.ensure<uint8_t>(hm.size());
-  cuda_check(cudaMemcpyAsync(dmask, hm.data(), hm.size(), cudaMemcpyHostToDevice, w.stream), "H2D masks");
   // o as exponent limbs on the device (only used when it does not fit 64 bits)
   const std::vector<uint32_t> ol = o.limbs(std::max<size_t>(1, (o.bitlen() + 31) / 32));
   uint32_t* dexp = nullptr;
@@ -801,6 +871,10 @@ void core_matmul_planes(KeyRec& k, Work& w, const uint32_t* x, size_t M, size_t 
     dexp = w.mm_exp.ensure<uint32_t>(ol.size() * 4);
     cuda_check(cudaMemcpyAsync(dexp, ol.data(), ol.size() * 4, cudaMemcpyHostToDevice, w.stream), "H2D exponent");
   }
+  if (k.kc.two_digit && matmul_two_digit(k, w, x, M, K, N, P, bit, o, dexp, ol.size(), out)) return;
+  const std::vector<uint8_t> hm = plane_masks(K, N, P, 8, bit);
+  uint8_t* dmask = w.mm_masks.ensure<uint8_t>(hm.size());
+  cuda_check(cudaMemcpyAsync(dmask, hm.data(), hm.size(), cudaMemcpyHostToDevice, w.stream), "H2D masks");
   const size_t per_row = hg::subset_table_bytes_per_row(k.S, (int)K);
   const size_t budget = (size_t)8 << 30;
   const size_t Rb = std::max<size_t>(1, std::min(M, budget / per_row));
@@ -813,12 +887,7 @@ void core_matmul_planes(KeyRec& k, Work& w, const uint32_t* x, size_t M, size_t 
                "matmul planes");
     if (!o.is_zero()) {
       cuda_check(hg::launch_row_products(k.S, k.kc, T, rows, (int)K, prod, w.stream), "row products");
-      core_inverse(k, w, prod, nullptr, prod, rows);
-      if (dexp)
-        cuda_check(hg::launch_pow_shared_bn(k.S, k.kc, prod, rows, dexp, (int)ol.size(), w.stream), "row power");
-      else
-        cuda_check(hg::launch_pow_shared(k.S, k.kc, prod, rows, o.low64(), w.stream), "row power");
-      cuda_check(hg::launch_scale_rows(k.S, k.kc, out, prod, r0, rows, (int)N, w.stream), "scale rows");
+      scale_by_offset(k, w, prod, r0, rows, N, o, dexp, ol.size(), out);
     }
   }
   // keep the host mask and exponent arrays alive until their copies have run
@@ -963,7 +1032,7 @@ bool build_sq_table(KeyRec& k) {
   cuda_check(hg::launch_sq_bases(S, kc, d + first, b, nullptr), "table bases");
   for (int p0 = 0; p0 < kc.npos; p0 += step)
     for (int lv = -1; lv < kc.w + (p0 == 0 ? 1 : 0); ++lv)
-      cuda_check(hg::launch_sq_level(S, kc, tab, iv, b, p0, lv < kc.w ? std::min(step, kc.npos - p0) : 1, lv, nullptr),
+      cuda_check(hg::launch_sq_level(S, kc, tab, iv, b, p0, (size_t)(lv < kc.w ? std::min(step, kc.npos - p0) : 1), lv, 0, nullptr),
                  "table level");
   cuda_check(cudaDeviceSynchronize(), "table build");
   kc.two_digit = 1;

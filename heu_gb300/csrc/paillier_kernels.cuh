@@ -143,8 +143,10 @@ cudaError_t launch_sq_encrypt(int S, const KeyConst& kc, const EncArgs& a, uint3
 // entries of npos positions from pos0, whose inverses are in `inv` (H limbs an
 // entry of those positions); level w multiplies position 0 by 2^(32 S).
 cudaError_t launch_sq_bases(int S, const KeyConst& kc, const uint32_t* first, uint32_t* bases, cudaStream_t st);
+// `subset`: the table's base entries are those of single bits already there,
+// and a level makes the other masks below 2^(level + 1) (sq_matmul.cu).
 cudaError_t launch_sq_level(int S, const KeyConst& kc, uint32_t* table, uint32_t* inv, const uint32_t* bases, int pos0,
-                            int npos, int level, cudaStream_t st);
+                            size_t npos, int level, int subset, cudaStream_t st);
 cudaError_t launch_add(int S, const KeyConst& kc, const uint32_t* a, const uint32_t* b, uint32_t* out,
                        size_t count, uint32_t* err, cudaStream_t st);
 cudaError_t launch_add_plain(int S, const KeyConst& kc, const uint32_t* a, const int64_t* p, int neg_p,
@@ -264,6 +266,21 @@ cudaError_t launch_pow_shared_bn(int S, const KeyConst& kc, uint32_t* v, size_t 
 cudaError_t launch_scale_rows(int S, const KeyConst& kc, uint32_t* out, const uint32_t* q, size_t r0, size_t rows,
                               int Ncols, cudaStream_t st);
 size_t subset_table_bytes_per_row(int S, int K);
+
+// MatMul of two-digit keys (sq_matmul.cu): chunks of b bases; per row nch =
+// ceil(K / b) chunks of 2^b - 1 entries of S limbs (T) and H limbs (inv), and
+// nch * b leaves of H limbs.
+int sq_matmul_chunk(size_t K, size_t N, size_t P);
+cudaError_t launch_mm_bases(int S, const KeyConst& kc, const uint32_t* x, size_t r0, size_t rows, int K, int b,
+                            uint32_t* T, uint32_t* leaves, uint32_t* err, cudaStream_t st);
+cudaError_t launch_mm_log(int S, const KeyConst& kc, size_t rows, int K, int b, uint32_t* T, const uint32_t* leaves,
+                          uint32_t* inv, cudaStream_t st);
+cudaError_t launch_half_up(int S, const KeyConst& kc, const uint32_t* lower, size_t lower_count, uint32_t* upper,
+                           cudaStream_t st);
+cudaError_t launch_half_down(int S, const KeyConst& kc, uint32_t* lower, size_t lower_count, const uint32_t* upper,
+                             cudaStream_t st);
+cudaError_t launch_mm_planes(int S, const KeyConst& kc, const uint32_t* T, const uint8_t* masks, size_t r0,
+                             size_t rows, int Ncols, int P, int K, int b, uint32_t* out, cudaStream_t st);
 
 // Occupancy-derived grid sizes (blocks) for the persistent kernels.
 int resident_blocks_mul(int S, int variant);

@@ -245,3 +245,54 @@ def test_mul_in_every_layout(edge_key, bits):
         for length in (1, 2, 3, 9, 301, 609, 1217, 2433, 4865, count):
             assert np.array_equal(key.mul(ct[:length], k[:length]), whole[:length]), (variant, length)
     autotune.set_config(key, cfg)
+
+
+@pytest.mark.parametrize("M,K,N,lo,hi", [
+    (1, 1, 1, 0, 2),  # one bit plane, one chunk
+    (2, 3, 1, -4, 4),
+    (3, 9, 2, 0, 1),  # all exponents 0
+    (1, 17, 24, -(2 ** 15), 2 ** 15),  # wide chunks, a ragged last one
+    (2, 5, 3, -(2 ** 63), 2 ** 63 - 1),  # 64 planes: the sum is taken below n on the way
+    (70, 2, 2, 0, 2 ** 20),  # no offset
+])
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("bits", [1024, 2048, 3072])
+def test_matmul_shapes(edge_key, bits, dense, M, K, N, lo, hi):
+    key, n, h_s, _, _ = edge_key(bits, dense)
+    n2, S = n * n, key.ct_limbs
+    R = pow(2, 32 * S, n2)
+    rng = np.random.default_rng(M * 100 + K)
+    x = [pow(h_s, 5 + i, n2) * (1 + i * n) % n2 for i in range(M * K)]
+    if K > 2:
+        x[1], x[2] = 1, n2 - 1
+    y = rng.integers(lo, hi, (K, N))
+    y[0, 0] = lo
+    got = key.matmul(hg.ints_to_limbs([v * R % n2 for v in x], S).reshape(M, K, S), y)
+    for i in range(0, M, max(1, M // 3)):
+        for j in range(N):
+            want = 1
+            for k in range(K):
+                want = want * pow(x[i * K + k], int(y[k, j]), n2) % n2
+            assert hg.limbs_to_ints(got[i, j])[0] == want * R % n2, (i, j)
+
+
+@pytest.mark.parametrize("bits", [1024, 2048])
+def test_matmul_with_bases_that_are_no_units(edge_key, bits):
+    """Zero and multiples of a prime have no inverse modulo n; their powers are
+    still defined for exponents >= 0, and an exponent below 0 is an error."""
+    key, n, h_s, p, q = edge_key(bits, False)
+    n2, S = n * n, key.ct_limbs
+    R = pow(2, 32 * S, n2)
+    x = [0, p, 7 * q, pow(h_s, 3, n2), n, 1]
+    y = np.array([[0, 1], [3, 0], [0, 2], [5, 9], [1, 0], [2, 3]])
+    limbs = hg.ints_to_limbs([v * R % n2 for v in x], S).reshape(1, 6, S)
+    got = hg.limbs_to_ints(key.matmul(limbs, y).reshape(2, S))
+    for j in range(2):
+        want = 1
+        for v, e in zip(x, y[:, j]):
+            want = want * pow(v, int(e), n2) % n2
+        assert got[j] == want * R % n2
+    with pytest.raises(hg.HgError):
+        key.matmul(limbs, -y)
+    with pytest.raises(hg.HgError):
+        key.matmul(hg.ints_to_limbs([n2] * 6, S).reshape(1, 6, S), y)
