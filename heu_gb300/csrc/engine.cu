@@ -177,6 +177,7 @@ struct KeyRec {
   DevBuf consts, sconsts, table, progs, fprogs;
   DevBuf sqconsts;            // two-digit encryption: e0 e1 rz (S each), rho2, nrho2 (H each)
   std::vector<uint32_t> hn;   // n (S/2 limbs)
+  hg::SquareInverse sqinv;    // the batch inverse's root modulo n^2
   hg::KeyConst kc{};
   hg::SecConst sc{};
   int grid_mul = 0;
@@ -198,6 +199,7 @@ struct KeyRec {
 // runs in stream order (and as a host node inside a captured CUDA graph).
 struct InvTask {
   const BN* N = nullptr;
+  const hg::SquareInverse* square = nullptr;  // of N = n^2, else null
   int S = 0;
   uint32_t* root = nullptr;  // pinned: S limbs of the root, then the kernels' error word
   uint32_t* z = nullptr;     // pinned: S limbs of the root's inverse, Montgomery form
@@ -215,7 +217,7 @@ void CUDART_CB inv_host_fn(void* p) {
     return;
   }
   // root = X*R; the tree's down-sweep wants X^-1 * R
-  if (!hg::mont_root_inverse(t->root, *t->N, S, t->z)) {
+  if (!(t->square ? t->square->root_inverse(t->root, t->z) : hg::mont_root_inverse(t->root, *t->N, S, t->z))) {
     if (t->status == 0) t->status = 1;
     for (size_t i = 0; i < S; ++i) t->z[i] = 0u;
   }
@@ -578,6 +580,7 @@ void core_inverse_async_raw(KeyRec& k, const uint32_t* in, const int64_t* sel, u
     if (sz == 1) break;
   }
   task.N = &k.N;
+  task.square = k.kc.two_digit ? &k.sqinv : nullptr;
   task.S = k.S;
   cuda_check(hg::launch_tree_leaves(k.S, k.kc, in, sel, count, tr, errp, st), "tree leaves");
   for (size_t l = 0; l + 1 < off.size(); ++l)
@@ -1035,6 +1038,13 @@ bool build_sq_table(KeyRec& k) {
       cuda_check(hg::launch_sq_level(S, kc, tab, iv, b, p0, (size_t)(lv < kc.w ? std::min(step, kc.npos - p0) : 1), lv, 0, nullptr),
                  "table level");
   cuda_check(cudaDeviceSynchronize(), "table build");
+  const BN R = BN(1).shl(32 * (size_t)S), ir2 = (ir * ir) % n;
+  k.sqinv.n = n;
+  k.sqinv.N = N;
+  k.sqinv.R2 = ((R % N) * (R % N)) % N;
+  k.sqinv.rh2 = R % n;
+  k.sqinv.rm2 = (((ir2 * ir2) % n) * BN(1).shl(128)) % n;  // rho^-4 2^128
+  k.sqinv.S = (size_t)S;
   kc.two_digit = 1;
   return true;
 }
