@@ -216,8 +216,13 @@ DecryptPlan decrypt_plan(int Sp, const SecConst& sc, size_t count) {
       pl.warps = (int)warps;
     }
   }
+  // up to two blocks a multiprocessor for decrypt_latency.cu: 2048 bits 1.01 ms
+  // to 76 ciphertexts and 1.41 ms for 152, where the layouts above take 1.71 and
+  // 1.72; 304 take 2.76 ms against 1.73.  3072 bits: 2.25 and 4.47 ms against
+  // 4.90; 1024 bits: 0.41 against 0.53 ms, but 0.60 for 300.
+  pl.latency = count <= (size_t)std::max(sms, 1);
   const size_t slots = ((size_t)1 << (sc.wd - 1)) + 1;
-  pl.table_words = (size_t)pl.warps * slots * 32 * (size_t)(H >> pl.logtc);
+  pl.table_words = pl.latency ? 0 : (size_t)pl.warps * slots * 32 * (size_t)(H >> pl.logtc);
   pl.handoff_words = pl.chunk * 2 * (size_t)H;
   return pl;
 }
@@ -230,17 +235,21 @@ cudaError_t launch_decrypt(int Sp, const KeyConst& kc, const SecConst& sc, const
   uint32_t* z = scratch + pl.table_words;
   for (size_t off = 0; off < count; off += pl.chunk) {
     const size_t n = std::min(pl.chunk, count - off);
-    cudaError_t e = cudaMemsetAsync(ctr, 0, sizeof(*ctr), st);
-    if (e != cudaSuccess) return e;
-    HG_DISPATCH_DEC(H, pl.logtc, {
-      DecPrimes<TC * L> pr;
-      std::copy(primes, primes + 2 * TC * L, &pr.n[0][0]);
-      const size_t items = 2 * ((n + SqLanes<TC, L>::IPW - 1) / SqLanes<TC, L>::IPW);
-      k_dec_pow<TC, L><<<(unsigned)std::min(items, (size_t)pl.warps), 32, 0, st>>>(pr, kc, sc, ct + off * 4 * H, n,
-                                                                                  scratch, z, err, ctr);
-    });
-    count_launches(1);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    if (pl.latency) {
+      if ((e = launch_dec_latency(H, kc, sc, ct + off * 4 * H, n, z, err, st)) != cudaSuccess) return e;
+    } else {
+      if ((e = cudaMemsetAsync(ctr, 0, sizeof(*ctr), st)) != cudaSuccess) return e;
+      HG_DISPATCH_DEC(H, pl.logtc, {
+        DecPrimes<TC * L> pr;
+        std::copy(primes, primes + 2 * TC * L, &pr.n[0][0]);
+        const size_t items = 2 * ((n + SqLanes<TC, L>::IPW - 1) / SqLanes<TC, L>::IPW);
+        k_dec_pow<TC, L><<<(unsigned)std::min(items, (size_t)pl.warps), 32, 0, st>>>(pr, kc, sc, ct + off * 4 * H, n,
+                                                                                    scratch, z, err, ctr);
+      });
+      count_launches(1);
+      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
     const unsigned blocks = (unsigned)((n + 15) / 16);
     switch (H) {
       case 16: k_dec_tail<2><<<blocks, 128, 0, st>>>(kc, sc, z, n, out_i64, out_ovf, out_mag, out_neg, cd, off); break;

@@ -1115,8 +1115,9 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
     // mod pr the power is 1 + (pr-1) n, so L is -n/pr mod pr
     const BN hp = BN::invmod(k->p - k->q % k->p, k->p), hq = BN::invmod(k->q - k->p % k->q, k->q);
     const BN pinvq = BN::invmod(k->p, k->q);
-    // p q pinvqR c1_p c1_q c2_p c2_q vz_p vz_q (H) | one_p one_q (Sp)
-    std::vector<uint32_t> hs2(2 * (size_t)Sp + 9 * (size_t)H);
+    // p q pinvqR c1_p c1_q c2_p c2_q vz_p vz_q (H) | one_p one_q (Sp) | fold_p fold_q
+    const size_t E = (size_t)hg::dec_latency_limbs(H), fold_words = E * (E + 1);
+    std::vector<uint32_t> hs2(2 * (size_t)Sp + 9 * (size_t)H + 2 * fold_words);
     auto put2 = [&](size_t at, const BN& v, size_t limbs) { v.to_limbs(hs2.data() + at, limbs); };
     put2(0, k->p, H);
     put2(H, k->q, H);
@@ -1136,6 +1137,22 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
       const BN rho = BN(1).shl(32 * ((size_t)H + 1)) % pr2;
       put2(9 * H + sd * Sp, rho % pr, H);
       put2(9 * H + sd * Sp + H, neg((rho / pr) % pr), H);
+      // c_k = 2^(28 (k - E)) from the top, a division by 2^28 each
+      uint32_t* fold = hs2.data() + 9 * (size_t)H + 2 * (size_t)Sp + sd * fold_words;
+      auto put28 = [E](uint32_t* at, const BN& v) {
+        std::vector<uint32_t> w(E + 1);
+        v.to_limbs(w.data(), w.size());
+        for (size_t j = 0; j < E; ++j)
+          at[j] = (uint32_t)((w[28 * j / 32] | (uint64_t)w[28 * j / 32 + 1] << 32) >> 28 * j % 32) & 0xfffffffu;
+      };
+      const uint32_t np = neg_inv32(pr.d[0]);
+      BN c(1);
+      for (size_t k = E; k-- > 0;) {
+        c = (c + pr * BN((uint32_t)c.low64() * np & 0xfffffffu)).shr(28);
+        put28(fold + k * E, c);
+      }
+      const BN rho28 = BN(1).shl(28 * E);
+      put28(fold + E * E, rho28 - BN::invmod(pr, rho28));
     }
     k->primes.assign(2 * (size_t)H, 0u);
     k->p.to_limbs(k->primes.data(), H);
@@ -1152,6 +1169,7 @@ int load_key(hg_ctx* ctx, uint32_t key_bits, const uint32_t* n_l, const uint32_t
       sc.c2[sd] = ds + (5 + sd) * H;
       sc.vz[sd] = ds + (7 + sd) * H;
       sc.one[sd] = ds + 9 * H + sd * Sp;
+      sc.fold[sd] = ds + 9 * H + 2 * Sp + sd * fold_words;
     }
     sc.np1[0] = neg_inv32(k->p.d[0]);
     sc.np1[1] = neg_inv32(k->q.d[0]);

@@ -62,6 +62,10 @@ struct SecConst {
   const uint32_t* c1[2];    // -hp*R1 mod p, -hq*R1 mod q  (Sp/2 limbs)
   const uint32_t* c2[2];    // -d*hp mod p, the same for q (Sp/2 limbs)
   const uint32_t* vz[2];    // z that stands for C = 0 mod p: L = -p^-1 mod R1
+  // decrypt_latency.cu, limbs of 28 bits, E = dec_latency_limbs(Sp/2):
+  // 2^(28 k) 2^(-28 E) mod p (or q) for k < E, E limbs each, then -p^-1 mod
+  // 2^(28 E)
+  const uint32_t* fold[2];
   // the batch kernel's exponentiation (sq_decrypt.cuh)
   const uint8_t* fprog[2];  // windows of p-1, q-1, highest first
   const uint32_t* one[2];   // digits of 2^(16 Sp + 32) mod p^2, q^2 (Sp limbs)
@@ -183,6 +187,7 @@ cudaError_t launch_sel_from_neg(const uint8_t* neg, int64_t* sel, size_t count, 
 // `primes`: p and q on the host (Sp/2 limbs each); `scratch` holds
 // decrypt_plan's table_words + handoff_words limbs.
 struct DecryptPlan {
+  bool latency = false;  // few ciphertexts: decrypt_latency.cu
   int logtc = 0;         // log2 of the lanes per chain
   int warps = 0;         // warps of the exponentiation launch
   size_t chunk = 0;      // ciphertexts per pair of launches
@@ -193,6 +198,9 @@ cudaError_t launch_decrypt(int Sp, const KeyConst& kc, const SecConst& sc, const
                            const DecryptPlan& pl, const uint32_t* ct, size_t count, int64_t* out_i64,
                            uint8_t* out_ovf, uint32_t* out_mag, uint8_t* out_neg, uint32_t* scratch, uint32_t* err,
                            unsigned long long* ctr, cudaStream_t st, const Codec& cd = Codec{});
+int dec_latency_limbs(int H);  // limbs of 28 bits of a digit
+cudaError_t launch_dec_latency(int H, const KeyConst& kc, const SecConst& sc, const uint32_t* ct, size_t count,
+                               uint32_t* z, uint32_t* err, cudaStream_t st);
 size_t decrypt_wave(int Sp);  // ciphertexts of one full wave of the widest layout
 // OU decryption over S-limb ciphertexts with Sp-limb p^2 arithmetic
 // (S, Sp) in {(64, 32), (128, 64), (128, 96)}.

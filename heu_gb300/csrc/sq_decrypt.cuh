@@ -94,19 +94,25 @@ __device__ __forceinline__ void dec_tail(const KeyConst& kc, const SecConst& sc,
   }
 }
 
-// x in Montgomery form -> digit 1 of the power in chain 1.
-template <int TC, int L, class Mod>
-__device__ __forceinline__ void dec_digit(uint32_t (&x)[L], const SecConst& sc, int side, const Mod& n, uint32_t np,
-                                          const SqLanes<TC, L>& g) {
-  sq_redc<TC, L>(x, x, n, np, g);
-  // digit 0 is 1, or a multiple of p where p divides c: such a c decrypts as
-  // it always did, through the value that stands for it
+// Digits of the power -> its digit 1 in chain 1: digit 0 is 1, or a multiple
+// of p where p divides c: such a c decrypts as it always did, through the
+// value that stands for it.
+template <int TC, int L>
+__device__ __forceinline__ void dec_check(uint32_t (&x)[L], const SecConst& sc, int side, const SqLanes<TC, L>& g) {
   uint32_t any = x[0] ^ (g.t == 0 ? 1u : 0u);
 #pragma unroll
   for (int j = 1; j < L; ++j) any |= x[j];
   const uint32_t mask = (1u << TC) - 1u;
   const bool zero = ((__ballot_sync(kFull, any != 0u) >> g.base) & mask) != 0u;
   if (zero) load_slice<L>(x, sc.vz[side] + g.t * L);
+}
+
+// x in Montgomery form -> digit 1 of the power in chain 1.
+template <int TC, int L, class Mod>
+__device__ __forceinline__ void dec_digit(uint32_t (&x)[L], const SecConst& sc, int side, const Mod& n, uint32_t np,
+                                          const SqLanes<TC, L>& g) {
+  sq_redc<TC, L>(x, x, n, np, g);
+  dec_check<TC, L>(x, sc, side, g);
 }
 
 // The exponentiation in the batch kernel: the two sides of a ciphertext sit in

@@ -4,6 +4,7 @@ whose primes (and so n and n^2) have nothing but ones in their top limbs."""
 
 import numpy as np
 import pytest
+import torch
 
 import heu_gb300 as hg
 from heu_gb300 import autotune
@@ -296,3 +297,30 @@ def test_matmul_with_bases_that_are_no_units(edge_key, bits):
         key.matmul(limbs, -y)
     with pytest.raises(hg.HgError):
         key.matmul(hg.ints_to_limbs([n2] * 6, S).reshape(1, 6, S), y)
+
+
+@pytest.mark.parametrize("dense", [False, True])
+@pytest.mark.parametrize("bits", [1024, 2048, 3072])
+def test_decrypt_few_and_many_agree(edge_key, bits, dense):
+    """Lengths on both sides of the one from which decryption no longer takes a
+    block per ciphertext and prime, with ciphertexts that are multiples of a
+    prime or not below n^2."""
+    key, n, _, p, _ = edge_key(bits, dense)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(3 * bits + dense)
+    count = 4 * sms + 1
+    m = rng.integers(-(2 ** 63), 2 ** 63 - 1, count)
+    r = rng.integers(0, 2 ** 32, (count, key.r_limbs), dtype=np.uint32)
+    ct = key.encrypt(m, r)
+    ct[0] = hg.ints_to_limbs([p * 12345], ct.shape[1])[0]
+    ct[1] = hg.ints_to_limbs([1], ct.shape[1])[0]
+    ct[2] = hg.ints_to_limbs([n * n - 1], ct.shape[1])[0]
+    want, want_ovf = key.decrypt(ct)
+    assert np.array_equal(want[3:], m[3:]) and not want_ovf[3:].any()
+    for length in (1, 2, 3, sms // 2 + 1, sms, sms + 1):
+        got, ovf = key.decrypt(ct[:length])
+        assert np.array_equal(got, want[:length]) and np.array_equal(ovf, want_ovf[:length]), length
+    ct[0] = hg.ints_to_limbs([n * n], ct.shape[1])[0]
+    for length in (1, sms + 1):
+        with pytest.raises(hg.HgError):
+            key.decrypt(ct[:length])
