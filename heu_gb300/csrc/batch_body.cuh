@@ -85,7 +85,7 @@ __device__ __forceinline__ void run_tile(const BatchJob& job, const BatchTile& t
       const size_t inst = wbase + lane_inst;
       const bool active = inst < end;
       __syncwarp();
-      sq_encrypt<TPI / 2, L, 1>(n, job.kc, a, (uint32_t*)job.out, active ? inst : end - 1, active, ysm, nullptr, err,
+      sq_encrypt<TPI / 2, L, 1, 1>(n, job.kc, a, (uint32_t*)job.out, active ? inst : end - 1, active, ysm, nullptr, err,
                                 sg);
     }
   } else if (job.op == kBatchEncrypt) {

@@ -16,29 +16,30 @@ struct Modulus {
   uint32_t n[H];
 };
 
-// A warp per group of ciphertexts, or kWarps warps that share its products.
+// A warp per group of ciphertexts, or kWarps warps of each of kBlocks blocks
+// (a cluster) that share its products.
 //
 // Bound: the fmaheavy pipe.  131,072 encryptions of 2048 bits at table window
 // 16 took 32.2 ms as 66 products modulo n^2 each; as 63 products by integers of
 // n's length and a tail of about 7 they take 17.4 ms.
-template <int TC, int L, int kWarps>
+template <int TC, int L, int kWarps, int kBlocks = 1>
 __global__ void __launch_bounds__(32 * kWarps)
     k_sq_encrypt(const __grid_constant__ Modulus<TC * L> mod, const __grid_constant__ KeyConst kc,
                  const __grid_constant__ EncArgs a, uint32_t* __restrict__ out, size_t count, uint32_t* err) {
   using G = SqLanes<TC, L>;
   extern __shared__ __align__(16) uint32_t enc_area[];
   const G g;
-  const size_t inst = (size_t)blockIdx.x * G::IPW + g.iw;
+  const size_t inst = (size_t)(blockIdx.x / kBlocks) * G::IPW + g.iw;
   const bool active = inst < count;
   const size_t i = active ? inst : count - 1;
   uint32_t* area = enc_area + (threadIdx.x >> 5) * kEncWords<TC, L>;
   uint32_t* carries = enc_area + kWarps * kEncWords<TC, L>;
   if constexpr (TC == 1) {
-    sq_encrypt<TC, L, kWarps>(mod.n, kc, a, out, i, active, area, carries, err, g);
+    sq_encrypt<TC, L, kWarps, kBlocks>(mod.n, kc, a, out, i, active, area, carries, err, g);
   } else {
     uint32_t n[L];
     load_slice<L>(n, kc.n + g.t * L);
-    sq_encrypt<TC, L, kWarps>(n, kc, a, out, i, active, area, carries, err, g);
+    sq_encrypt<TC, L, kWarps, kBlocks>(n, kc, a, out, i, active, area, carries, err, g);
   }
 }
 
@@ -73,6 +74,24 @@ constexpr size_t enc_smem() {
   }
 
 constexpr int kShareWarps = 8;
+constexpr int kClusterWarps = 4;  // a warp for each scheduler
+
+template <int TC, int L, int kBlocks>
+cudaError_t launch_cluster(const Modulus<TC * L>& m, const KeyConst& kc, const EncArgs& a, uint32_t* out, size_t count,
+                           uint32_t* err, cudaStream_t st) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = kBlocks;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)count * kBlocks);
+  cfg.blockDim = dim3(32 * kClusterWarps);
+  cfg.dynamicSmemBytes = enc_smem<TC, L, kClusterWarps>();
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_sq_encrypt<TC, L, kClusterWarps, kBlocks>, m, kc, a, out, count, err);
+}
 
 // ---------------------------------------------------------------------------
 // tables
@@ -228,10 +247,25 @@ cudaError_t launch_sq_encrypt(int S, const KeyConst& kc, const EncArgs& a, uint3
   if (count == 0) return cudaSuccess;
   const int H = S / 2;
   const double scheds = 4.0 * sm_count();
-  // Shares: several warps on each ciphertext while that leaves schedulers with
-  // at most four warps, where the chain of products and not the pipe sets the
-  // time.  One ciphertext (2048 bits, window 12) takes 0.083 ms with 8 warps
-  // against 0.306 ms with one.
+  // Shares: several warps on each ciphertext, while the chain of products and
+  // not the pipe sets the time: over the multiprocessors of a cluster up to two
+  // warps a scheduler (more in one multiprocessor only slow each other down),
+  // then in one block up to four.  One ciphertext (2048 bits, window 12) takes
+  // 0.053 ms with 32 warps in 8 blocks, 0.059 with 16 in 4, 0.081 with 8 in one
+  // and 0.306 with one; 76 take 0.073 ms with 16 and 0.081 with 8; of 3072
+  // bits one takes 0.088, 0.103 and 0.173 ms with 32, 16 and 8.
+  for (int blocks = 8; blocks > 2; blocks >>= 1) {
+    if ((double)count * blocks * kClusterWarps > 2.0 * scheds) continue;
+    HG_DISPATCH_SQ16(H, {
+      Modulus<TC * L> m;
+      std::copy(kc.hn, kc.hn + H, m.n);
+      const cudaError_t e = blocks == 8 ? launch_cluster<TC, L, 8>(m, kc, a, out, count, err, st)
+                                        : launch_cluster<TC, L, 4>(m, kc, a, out, count, err, st);
+      if (e != cudaSuccess) return e;
+    });
+    count_launches(1);
+    return cudaGetLastError();
+  }
   for (int warps = kShareWarps; warps > 1; warps >>= 1) {
     if ((double)count * warps > 4.0 * scheds) continue;
     HG_DISPATCH_SQ16(H, {

@@ -10,6 +10,8 @@
 //   c = (P0 - P1 n)(1 - (sum y - m) n) = P0 - (P1 + P0 (sum y - m)) n.
 // y is stored times rho, so the last product of digits is one reduction.
 #pragma once
+#include <cooperative_groups.h>
+
 #include "paillier_ops.cuh"
 #include "sqmod.cuh"
 
@@ -65,17 +67,19 @@ __device__ __forceinline__ bool enc_plain(uint32_t (&A)[L], bool& neg, const Key
   return !(too_big || bad);
 }
 
-// One encryption per group of 2 TC lanes by kWarps warps of a block: warp w
-// multiplies the w-th share of the entries and warp 0 combines the shares, so
-// a short batch's chain of products is 1 / kWarps as long.  `area`: the warp's
-// kEncWords, `areas` those of warp 0 (kWarps > 1), `carries` 32 words a warp.
-template <int TC, int L, int kWarps, class Mod>
+// One encryption per group of 2 TC lanes by kWarps warps of each block of a
+// cluster of kBlocks: warp w multiplies the w-th share of the entries and warp 0
+// combines the shares, so a short batch's chain of products is shorter.
+// `area`: the warp's kEncWords, `carries` 32 words a warp.
+template <int TC, int L, int kWarps, int kBlocks, class Mod>
 __device__ __forceinline__ void sq_encrypt(const Mod& n, const KeyConst& kc, const EncArgs& a,
                                            uint32_t* __restrict__ out, size_t i, bool active, uint32_t* area,
                                            uint32_t* carries, uint32_t* err, const SqLanes<TC, L>& g) {
   constexpr int H = TC * L, S = 2 * H, kDigit = SqLanes<TC, L>::kDigit, V = SqLanes<TC, L>::kVec;
   const uint32_t np = kc.npn;
-  const int warp = kWarps > 1 ? (int)(threadIdx.x >> 5) : 0;
+  constexpr int kShares = kWarps * kBlocks;
+  const int slot = kWarps > 1 ? (int)(threadIdx.x >> 5) : 0;
+  const int warp = kBlocks > 1 ? (int)(blockIdx.x % kBlocks) * kWarps + slot : slot;
   const size_t ent = (size_t)((1u << kc.w) - 1u);
   const uint32_t* ri = a.r + i * kc.rlimbs;
   // entry e: the table's for digit position e, one of the identity for a zero
@@ -102,8 +106,8 @@ __device__ __forceinline__ void sq_encrypt(const Mod& n, const KeyConst& kc, con
   };
   uint32_t* sum = g.limb(area + 4 * kDigit, 0, 0);  // of the y, chain 1's slices
   const int total = kc.npos + (a.mode == EncMode::kRandomize ? 1 : 0);
-  int e = kWarps > 1 ? total * warp / kWarps : 0;
-  const int end = kWarps > 1 ? total * (warp + 1) / kWarps : total;
+  int e = kShares > 1 ? total * warp / kShares : 0;
+  const int end = kShares > 1 ? total * (warp + 1) / kShares : total;
   uint32_t x[L], carry = 0u;
   if (a.mode == EncMode::kRandomize && warp == 0) {
     const bool ok = raw_below<TC, L>(a.ct_in + i * S, kc.N);
@@ -153,15 +157,30 @@ __device__ __forceinline__ void sq_encrypt(const Mod& n, const KeyConst& kc, con
     __syncwarp();
     sq_pass<TC, L, false>(x, x, g.limb(cur, 0, 0), 0u, 0u, x, nullptr, n, np, g);
   }
-  if constexpr (kWarps > 1) {
-    // shares as a tree: warp w takes warp w + d's digits and sum
+  if constexpr (kShares > 1) {
+    // shares as a tree: warp w takes warp w + d's digits and sum, from another
+    // block's shared memory where d reaches beyond its own
+    namespace cg = cooperative_groups;
 #pragma unroll 1
-    for (int d = 1; d < kWarps; d <<= 1) {
-      sq_stage<TC, L>(area, x, true, g);
-      carries[warp * 32 + g.lane] = carry;
-      __syncthreads();
+    for (int d = 1; d < kShares; d <<= 1) {
+      if (warp % d == 0) {
+        sq_stage<TC, L>(area, x, true, g);
+        carries[slot * 32 + g.lane] = carry;
+      }
+      if (kBlocks > 1 && d >= kWarps)
+        cg::this_cluster().sync();
+      else
+        __syncthreads();
       if (warp % (2 * d) == 0) {
         uint32_t* other = area + d * kEncWords<TC, L>;
+        uint32_t* other_carries = carries + (slot + d) * 32;
+        if constexpr (kBlocks > 1) {
+          if (d >= kWarps) {
+            const unsigned rank = (unsigned)((warp + d) / kWarps);
+            other = cg::this_cluster().map_shared_rank(area, rank);
+            other_carries = cg::this_cluster().map_shared_rank(carries + slot * 32, rank);
+          }
+        }
         if (g.c == 1) {
           uint32_t s[L], y[L];
           sq_get<TC, L>(s, sum, g);
@@ -169,7 +188,7 @@ __device__ __forceinline__ void sq_encrypt(const Mod& n, const KeyConst& kc, con
           s[0] = add_cc(s[0], y[0]);
 #pragma unroll
           for (int j = 1; j < L; ++j) s[j] = addc_cc(s[j], y[j]);
-          carry = addc(carry, carries[(warp + d) * 32 + g.lane]);
+          carry = addc(carry, other_carries[g.lane]);
           sq_put<TC, L>(sum, s, g);
         }
         uint32_t y0[L];
@@ -177,8 +196,9 @@ __device__ __forceinline__ void sq_encrypt(const Mod& n, const KeyConst& kc, con
         sq_get<TC, L>(y0, g.limb(other, 0, 0), g);
         sq_pass<TC, L, true>(x, x, g.limb(area, 0, 0), 0u, 0u, y0, g.limb(area, 1, 0), n, np, g);
       }
-      __syncthreads();
     }
+    // the other blocks' shared memory has been read
+    if constexpr (kBlocks > 1) cg::this_cluster().sync();
     if (warp != 0) return;
   }
   // sum - m rho, then X1 += X0 * sum

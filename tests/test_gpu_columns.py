@@ -324,3 +324,24 @@ def test_decrypt_few_and_many_agree(edge_key, bits, dense):
     for length in (1, sms + 1):
         with pytest.raises(hg.HgError):
             key.decrypt(ct[:length])
+
+
+@pytest.mark.parametrize("window", [5, 12])
+@pytest.mark.parametrize("bits", [1024, 2048, 3072])
+def test_encrypt_few_and_many_agree(gpu_ctx, edge_key, bits, window):
+    """Lengths on both sides of those from which an encryption is shared by
+    fewer blocks, against the same values in a longer call."""
+    _, n, h_s, p, q = edge_key(bits, True)
+    key = gpu_ctx.load_key(bits, n, h_s, p, q, table_window=window)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(bits + window)
+    count = 16 * sms + 1
+    m = rng.integers(-(2 ** 63), 2 ** 63 - 1, count)
+    r = _randomness(key, rng, count)
+    ct, zero = key.encrypt(m, r), key.encrypt_zero(r)
+    again = key.randomize(ct, r[::-1].copy())
+    for length in (1, 2, sms // 4, sms // 4 + 1, sms // 2, sms // 2 + 1, 2 * sms, 2 * sms + 1):
+        assert np.array_equal(key.encrypt(m[:length], r[:length]), ct[:length]), length
+        assert np.array_equal(key.encrypt_zero(r[-length:]), zero[-length:]), length
+        assert np.array_equal(key.randomize(ct[:length], r[::-1][:length].copy()), again[:length]), length
+    key.free()
