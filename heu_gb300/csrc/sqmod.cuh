@@ -200,7 +200,11 @@ __device__ __forceinline__ void sq_settle(uint32_t (&x)[L], const uint32_t (&Ev)
 // limbs) 85.0, 81.9 and 80.5 ms, 65,536 of 2048 bits with 16 limbs a lane 97.4,
 // 91.0 and 87.7 ms.  (Multipliers in 16-byte loads then took 1 to 3% off each.)
 template <int TC, int L>
+#ifdef HG_SQ_UNROLL  // batch_v0.cu
+constexpr int kSqUnroll = HG_SQ_UNROLL;
+#else
 constexpr int kSqUnroll = TC == 1 && L == 32 ? 8 : 16;
+#endif
 
 // Layouts whose passes run sq_step_early: the widest of the primes' lengths,
 // which only few ciphertexts take.  8 CRT decryptions of 2048 bits (16 lanes a
