@@ -32,9 +32,8 @@ struct BatchTile {
   uint32_t pad;
 };
 
-// (threads per instance) for n^2 with S limbs and (threads per side) for p^2
-// with SP limbs, per variant; V = 0 / 1 must match HG_DISPATCH_SV /
-// HG_DISPATCH_SPV, V = 2 (latency layout) HG_DISPATCH_SL / HG_DISPATCH_SPL.
+// Lanes of an instance for n^2 with S limbs, and of a side of a decryption (two
+// chains) for p^2 with SP limbs, per variant; V = 2: the latency layout.
 __host__ __device__ constexpr int tpi_for(int S, int V) {
   return V == 2 ? 32 : S == 64 ? (V ? 8 : 4) : S == 128 ? (V ? 4 : 8) : (V ? 8 : 16);
 }

@@ -5,14 +5,14 @@
 //
 // One launch runs a whole batch of jobs of different key sizes (1024, 2048,
 // 3072 bits) and operations (encrypt, decrypt, add, scalar mul).  The host
-// cuts every job into tiles of a few warp passes and orders them by cost
-// (most expensive first); each warp repeatedly takes the next tile from a
-// device counter and runs the per-ciphertext body of paillier_ops.cuh for
-// the tile's key size.  All key sizes of one launch use the (threads per
-// instance, limbs per thread) layouts of variant set V (tpi_for / tp_for):
-// V = 0 and 1 are throughput layouts the autotuner picks from, V = 2 the
-// latency layout (a whole warp per instance mod n^2, a half warp per side
-// mod p^2) that short requests run in.
+// cuts every job into tiles of one warp pass (additions: four) and orders them
+// by cost (most expensive first); each warp repeatedly takes the next tile from
+// a device counter and runs the per-ciphertext body for the tile's key size:
+// two digits modulo n (sq_encrypt.cuh, sq_mul.cuh) or a prime (sq_decrypt.cuh),
+// additions modulo n^2 (paillier_ops.cuh).  All key sizes of one launch use the
+// layouts of variant set V (tpi_for / tp_for): V = 0 and 1 are throughput
+// layouts the autotuner picks from, V = 2 the latency layout (a whole warp per
+// instance, a half warp per side of a decryption) that short requests run in.
 #pragma once
 #include <algorithm>
 

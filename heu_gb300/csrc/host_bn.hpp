@@ -420,7 +420,7 @@ inline bool mont_root_inverse(const uint32_t* xr, const BN& N, size_t S, uint32_
 // inverse modulo n, of half the length and a quarter of the steps, lifted once
 // (Hensel / Newton): with x t0 = R^2 mod n,
 //   t = t0 + n ((R^2 - x t0) / n) x^-1 mod n,  and then x t = R^2 mod n^2.
-// One 4096-bit inverse on the GPU machine's cores takes 137 us against 344.
+// One 4096-bit inverse on Grace cores takes 137 us against 344.
 struct SquareInverse {
   BN n, N;
   BN R2;   // R^2 mod N, R = 2^(32 S)
