@@ -305,8 +305,9 @@ __device__ __forceinline__ void sq_redc_step(uint32_t (&Ev)[L], uint32_t (&Od)[L
 }
 
 // Digits of W * 2^(-32 (kWide - H + 1)) for a raw number W of kWide >= H
-// limbs (`src`, 16-byte aligned, this instance's): chain 0 takes the limbs in
-// from below its top as it reduces.  kWide = H: a reduction of W by rho.
+// limbs (`src`, this instance's; a caller's array, of which no more than 8-byte
+// alignment is asked): chain 0 takes the limbs in from below its top as it
+// reduces.  kWide = H: a reduction of W by rho.
 template <int TC, int L, int kWide, class Mod>
 __device__ __forceinline__ void sq_from_raw(uint32_t (&z)[L], const uint32_t* __restrict__ src, const Mod& n,
                                             uint32_t np, const SqLanes<TC, L>& g) {
@@ -320,11 +321,15 @@ __device__ __forceinline__ void sq_from_raw(uint32_t (&z)[L], const uint32_t* __
   }
   uint32_t ov = 0u, c1 = 0u;
   const bool taker = g.c == 0 && g.t == TC - 1;
-  const uint4* q = reinterpret_cast<const uint4*>(src + H);
-  uint4 v = taker ? q[0] : make_uint4(0u, 0u, 0u, 0u);
+  auto limbs = [&](int i) {
+    const uint2* q = reinterpret_cast<const uint2*>(src + H + i);
+    const uint2 lo = q[0], hi = q[1];
+    return make_uint4(lo.x, lo.y, hi.x, hi.y);
+  };
+  uint4 v = taker ? limbs(0) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll 1
   for (int i = 0; i < kIn; i += 4) {
-    const uint4 nx = (taker && i + 4 < kIn) ? q[i / 4 + 1] : make_uint4(0u, 0u, 0u, 0u);
+    const uint4 nx = (taker && i + 4 < kIn) ? limbs(i + 4) : make_uint4(0u, 0u, 0u, 0u);
     sq_redc_step<TC, L>(E, O, ov, c1, n, np, v.x, g);
     sq_redc_step<TC, L>(O, E, ov, c1, n, np, v.y, g);
     sq_redc_step<TC, L>(E, O, ov, c1, n, np, v.z, g);
