@@ -65,6 +65,16 @@ struct Lat {
   static constexpr size_t smem(size_t slots, size_t steps) {
     return ((size_t)kTab + slots * 2 * RP) * 4 + (steps + 2) * 4;
   }
+  // The most that any key takes: a program of w-bit windows has a squaring a bit
+  // and a product for every w of them at most (build_prog).
+  static constexpr size_t smem_bound() {
+    size_t most = 0;
+    for (size_t w = kMinDecWindow; w <= kMaxDecWindow; ++w) {
+      const size_t ntab = (size_t)1 << (w - 1), b = smem(ntab + 1, ntab + 32 * H + 32 * H / w + 1);
+      most = most > b ? most : b;
+    }
+    return most;
+  }
 };
 
 // A quarter of columns k and k + 1 of a product: the NR rows at `a` by the NR + 1
@@ -315,8 +325,13 @@ cudaError_t launch_dec_latency(int H_, const KeyConst& kc, const SecConst& sc, c
   const size_t ntab = (size_t)1 << (sc.wd - 1), steps = ntab + (size_t)sc.prog_len;
   HG_DISPATCH_LAT(H_, {
     const size_t smem = Lat<H>::smem(ntab + 1, steps);
+    constexpr size_t kBound = Lat<H>::smem_bound();
+    static_assert(kBound <= 227 * 1024, "shared memory");
+    if (smem > kBound) return cudaErrorInvalidValue;
     if (smem > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(k_dec_latency<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      // The limit is the function's, for all threads and keys: every call sets it to
+      // the same bound, so that none takes another's away before its launch.
+      const cudaError_t e = cudaFuncSetAttribute(k_dec_latency<H>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBound);
       if (e != cudaSuccess) return e;
     }
     k_dec_latency<H><<<(unsigned)(2 * count), 32 * Lat<H>::kWarps, smem, st>>>(kc, sc, ct, z, err);

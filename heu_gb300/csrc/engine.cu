@@ -2422,7 +2422,7 @@ static void apply_config(KeyRec& k, const hg_key_config& c) {
   if (c.variant < 0 || c.variant > 1 || c.dec_variant < 0 || c.dec_variant > 1)
     fail(HG_ERR_INVALID, "variant must be 0 or 1");
   if (c.mul_window < 2 || c.mul_window > 6) fail(HG_ERR_INVALID, "mul_window must be in [2, 6]");
-  if (c.dec_window < 2 || c.dec_window > 7) fail(HG_ERR_INVALID, "dec_window must be in [2, 7]");
+  if (c.dec_window < hg::kMinDecWindow || c.dec_window > hg::kMaxDecWindow) fail(HG_ERR_INVALID, "dec_window must be in [2, 7]");
   cuda_check(cudaDeviceSynchronize(), "sync");
   k.kc.variant = c.variant;
   k.grid_mul = hg::resident_blocks_mul(k.S, c.variant);

@@ -96,6 +96,8 @@ struct OuConst {
   int Sp;                 // 32-bit limbs of the p^2 arithmetic
 };
 
+// Window bits that a key's decryption may be configured with.
+constexpr int kMinDecWindow = 2, kMaxDecWindow = 7;
 // Window bits of the batch kernel's decryption (SecConst::fprog).
 constexpr int kBatchDecWindow = 5;
 // Table entries of a warp's scalar multiplication (sq_mul.cuh): the powers 0 ..

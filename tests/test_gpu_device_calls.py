@@ -1,13 +1,14 @@
 """What a device call asks of its caller besides its values: the alignment of
-its arrays."""
+its arrays, and that calls of other threads and keys leave it alone."""
 
 import ctypes
+import threading
 
 import numpy as np
 import pytest
 import torch
 
-from heu_gb300 import capi
+from heu_gb300 import autotune, capi
 
 pytestmark = pytest.mark.gpu
 
@@ -55,3 +56,48 @@ def test_few_ciphertexts_at_eight_byte_alignment(gpu_ctx, gpu_key, bits, seed):
         assert torch.equal(odd, want), count
         assert np.array_equal(out.cpu().numpy(), m) and not ovf.any(), count
         assert not held[:2].any()
+
+
+def test_few_decryptions_of_two_keys_from_many_threads(gpu_ctx, gpu_key):
+    """Two 3072-bit keys with the widest window, whose exponent programs differ
+    in length and so in the shared memory that a launch for few ciphertexts asks
+    for: calls of one do not take the other's limit away."""
+    bits = 3072
+    p, q = 2 ** (bits // 2) - 3453, 2 ** (bits // 2) - 4977  # exponents of ones: the longest programs
+    n = p * q
+    dense = gpu_ctx.load_key(bits, n, pow(n - 9, n, n * n), p, q, table_window=5)
+    plain, _, _ = gpu_key(bits, 2)
+    dev = torch.device("cuda", 0)
+    rng = np.random.default_rng(1)
+    saved = autotune.get_config(plain)
+    work, failed = [], []
+    try:
+        for key in (dense, plain):
+            autotune.set_config(key, dict(autotune.get_config(key), dec_window=7))
+            m, dm, dr = _column(key, rng, 1, dev)
+            ct = torch.empty((1, key.ct_limbs), dtype=torch.int32, device=dev)
+            torch.cuda.synchronize()
+            capi.check(key.lib.hg_dev_encrypt(key.ctx.handle, key.id, _p(dm), _p(dr), _p(ct), 1, None))
+            capi.check(key.lib.hg_dev_check(key.ctx.handle))
+            for _ in range(4):
+                work.append((key, m[0], ct, torch.zeros(1, dtype=torch.int64, device=dev),
+                             torch.zeros(1, dtype=torch.uint8, device=dev), torch.cuda.Stream()))
+        torch.cuda.synchronize()
+
+        def calls(key, m, ct, out, ovf, stream):
+            s = ctypes.c_void_p(stream.cuda_stream)
+            for _ in range(300):
+                if key.lib.hg_dev_decrypt(key.ctx.handle, key.id, _p(ct), _p(out), _p(ovf), 1, s):
+                    failed.append(key.lib.hg_last_error())
+
+        threads = [threading.Thread(target=calls, args=w) for w in work]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        assert not failed, (len(failed), failed[0])
+        assert all(int(out) == m for _, m, _, out, _, _ in work)
+    finally:
+        autotune.set_config(plain, saved)
+        dense.free()
