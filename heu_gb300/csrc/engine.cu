@@ -505,7 +505,7 @@ void decrypt_crt(KeyRec& k, Work& w, const uint32_t* ct, int64_t* m, uint8_t* ov
   if (!k.secret) fail(HG_ERR_NO_SECRET, "key has no secret part");
   if (count == 0) return;
   const hg::DecryptPlan pl = hg::decrypt_plan(k.Sp, k.sc, count);
-  uint32_t* scratch = w.scratch.ensure<uint32_t>((pl.table_words + pl.handoff_words) * 4);
+  uint32_t* scratch = w.scratch.ensure<uint32_t>(hg::decrypt_scratch_words(k.Sp, k.sc) * 4);
   cuda_check(hg::launch_decrypt(k.Sp, k.kc, k.sc, k.primes.data(), pl, ct, count, m, ovf, mag, neg, scratch, w.errp(),
                                 w.ctrp(), w.stream, cd),
              "decrypt launch");
@@ -628,8 +628,8 @@ void core_inverse(KeyRec& k, Work& w, const uint32_t* in, const int64_t* sel, ui
 void mul_powers(KeyRec& k, Work& w, const uint32_t* a, const int64_t* kk, uint32_t* out, size_t count) {
   if (count == 0) return;
   if (k.kc.two_digit) {
-    const hg::MulPlan pl = hg::mul_plan(k.S, k.kc, k.wm, count);
-    uint32_t* scratch = w.scratch.ensure<uint32_t>(pl.scratch_words * 4);
+    const hg::MulPlan pl = hg::mul_plan(k.S, k.kc, count);
+    uint32_t* scratch = w.scratch.ensure<uint32_t>(hg::mul_scratch_words(k.S, k.wm) * 4);
     cuda_check(hg::launch_sq_mul(k.S, k.kc, pl, a, kk, out, count, scratch, k.wm, w.errp(), w.ctrp(), w.stream),
                "mul launch");
     return;

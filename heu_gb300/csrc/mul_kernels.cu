@@ -76,7 +76,7 @@ int resident_warps(int H, int logtc) {
 
 }  // namespace
 
-MulPlan mul_plan(int S, const KeyConst& kc, int wm, size_t count) {
+MulPlan mul_plan(int S, const KeyConst& kc, size_t count) {
   const int H = S / 2;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -104,8 +104,16 @@ MulPlan mul_plan(int S, const KeyConst& kc, int wm, size_t count) {
       pl.warps = (int)warps;
     }
   }
-  pl.scratch_words = (size_t)pl.warps * mul_slots(wm) * 32 * (size_t)(H >> pl.logtc);
   return pl;
+}
+
+// The most that any count's plan takes, as decrypt_scratch_words.
+size_t mul_scratch_words(int S, int wm) {
+  const int H = S / 2;
+  size_t words = 0;
+  for (int l = 1; l < 5; ++l)
+    if (has_layout(H, l)) words = std::max(words, (size_t)resident_warps(H, l) * mul_slots(wm) * 32 * (size_t)(H >> l));
+  return words;
 }
 
 cudaError_t launch_sq_mul(int S, const KeyConst& kc, const MulPlan& pl, const uint32_t* a, const int64_t* k,

@@ -162,13 +162,14 @@ cudaError_t launch_add_plain(int S, const KeyConst& kc, const uint32_t* a, const
 cudaError_t launch_mul(int S, const KeyConst& kc, const uint32_t* a, const int64_t* k, uint32_t* out,
                        size_t count, uint32_t* scratch, int wm, uint32_t* err, int grid, unsigned long long* ctr,
                        cudaStream_t st);
-// Mul of two-digit keys (mul_kernels.cu) over mul_plan's scratch.
+// Mul of two-digit keys (mul_kernels.cu); `scratch` holds mul_scratch_words
+// limbs.
 struct MulPlan {
   int logtc = 1;  // log2 of the lanes per chain
   int warps = 0;
-  size_t scratch_words = 0;
 };
-MulPlan mul_plan(int S, const KeyConst& kc, int wm, size_t count);
+MulPlan mul_plan(int S, const KeyConst& kc, size_t count);
+size_t mul_scratch_words(int S, int wm);
 cudaError_t launch_sq_mul(int S, const KeyConst& kc, const MulPlan& pl, const uint32_t* a, const int64_t* k,
                           uint32_t* out, size_t count, uint32_t* scratch, int wm, uint32_t* err,
                           unsigned long long* ctr, cudaStream_t st);
@@ -187,15 +188,16 @@ cudaError_t launch_sel_from_neg(const uint8_t* neg, int64_t* sel, size_t count, 
 // With cd.kind != kCodecNone out_i64 receives the decoded values (int64 or
 // double, per cd.kind) and cd.out1 the second slot of batch kinds.
 // `primes`: p and q on the host (Sp/2 limbs each); `scratch` holds
-// decrypt_plan's table_words + handoff_words limbs.
+// decrypt_scratch_words limbs.
 struct DecryptPlan {
   bool latency = false;  // few ciphertexts: decrypt_latency.cu
   int logtc = 0;         // log2 of the lanes per chain
   int warps = 0;         // warps of the exponentiation launch
   size_t chunk = 0;      // ciphertexts per pair of launches
-  size_t table_words = 0, handoff_words = 0;
+  size_t table_words = 0;  // of the scratch, before the digits handed over
 };
 DecryptPlan decrypt_plan(int Sp, const SecConst& sc, size_t count);
+size_t decrypt_scratch_words(int Sp, const SecConst& sc);
 cudaError_t launch_decrypt(int Sp, const KeyConst& kc, const SecConst& sc, const uint32_t* primes,
                            const DecryptPlan& pl, const uint32_t* ct, size_t count, int64_t* out_i64,
                            uint8_t* out_ovf, uint32_t* out_mag, uint8_t* out_neg, uint32_t* scratch, uint32_t* err,

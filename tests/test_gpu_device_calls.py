@@ -1,5 +1,6 @@
 """What a device call asks of its caller besides its values: the alignment of
-its arrays, and that calls of other threads and keys leave it alone."""
+its arrays, that calls of other threads and keys leave it alone, and what a
+first call allocates."""
 
 import ctypes
 import threading
@@ -101,3 +102,59 @@ def test_few_decryptions_of_two_keys_from_many_threads(gpu_ctx, gpu_key):
     finally:
         autotune.set_config(plain, saved)
         dense.free()
+
+
+def _held(lib):
+    held = ctypes.c_size_t()
+    capi.check(lib.hg_probe_set_alloc_limit(0, ctypes.byref(held)))
+    return held.value
+
+
+@pytest.mark.parametrize("bits,seed", [(1024, 1), (2048, 0), (3072, 2)])
+def test_a_short_call_leaves_room_for_a_long_one(gpu_key, bits, seed):
+    """A stream's first decryption allocates what one of any length takes, and
+    its first Mul all but the batch inverse's tree: a longer decryption after a
+    short one neither allocates nor frees, so it may be captured, and what was
+    captured before it stays valid."""
+    dev = torch.device("cuda", 0)
+    key, _, _ = gpu_key(bits, seed)
+    lib, h = key.lib, key.ctx.handle
+    count = 30000 if bits < 3072 else 6000
+    rng = np.random.default_rng(bits)
+    m, dm, dr = _column(key, rng, count, dev)
+    ct = torch.empty((count, key.ct_limbs), dtype=torch.int32, device=dev)
+    prod, ones = torch.empty_like(ct), torch.ones(count, dtype=torch.int64, device=dev)
+    out, ovf = torch.zeros(count, dtype=torch.int64, device=dev), torch.empty(count, dtype=torch.uint8, device=dev)
+    stream, other = torch.cuda.Stream(), torch.cuda.Stream()
+    s, s2 = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p(other.cuda_stream)
+    torch.cuda.synchronize()
+    capi.check(lib.hg_dev_encrypt(h, key.id, _p(dm), _p(dr), _p(ct), count, s))
+    torch.cuda.synchronize()
+
+    def decrypt(n):
+        capi.check(lib.hg_dev_decrypt(h, key.id, _p(ct), _p(out), _p(ovf), n, s))
+
+    decrypt(1)
+    base = _held(lib)
+    for n in (2, 700, 2500, count):
+        decrypt(n)
+        assert _held(lib) == base, n
+    capi.check(lib.hg_dev_mul(h, key.id, _p(ct), _p(ones), _p(prod), 3, s2))
+    base = _held(lib)
+    capi.check(lib.hg_dev_mul(h, key.id, _p(ct), _p(ones), _p(prod), count, s2))
+    tree = (2 * count + 64) * key.ct_limbs * 4
+    assert base <= _held(lib) <= base + tree
+    torch.cuda.synchronize()
+    assert torch.equal(prod, ct)
+    graphs = []
+    for n in (5, count):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=stream):
+            decrypt(n)
+        graphs.append((n, g))
+    for n, g in graphs[::-1]:
+        out.zero_()
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        assert np.array_equal(out[:n].cpu().numpy(), m[:n]) and not out[n:].any()
