@@ -1,10 +1,10 @@
 """Project autotuner front end: runs the engine's hg_autotune sweep for a key
 and persists the chosen configuration per device and key size as JSON.
 
-The sweep (C++, in the engine) times encrypt and scalar mul for both
-(threads per ciphertext, limbs per thread) variants and mul windows 2..6,
-and CRT decrypt for both mod-p^2 variants and windows 4..7, then applies the
-fastest.  The configuration never changes results, only speed.
+The sweep (C++, in the engine) times scalar mul with windows 2..6 and CRT
+decrypt with windows 4..7, then applies the fastest; layouts follow the length
+of each call and are not tuned.  The configuration never changes results, only
+speed.
 """
 
 import ctypes

@@ -53,7 +53,7 @@ class Batch:
 
     def set_variant(self, variant):
         """0 or 1: every job in that layout variant set; PER_KEY: each job in
-        its key's tuned layout, one persistent launch per set in use."""
+        its key's configured layout, one persistent launch per set in use."""
         capi.check(self.lib.hg_batch_set_variant(self.handle, variant))
 
     def run(self, stream=None, graph=False):

@@ -205,7 +205,7 @@ DecryptPlan decrypt_plan(int Sp, const SecConst& sc, size_t count) {
   DecryptPlan pl;
   pl.chunk = std::min(count, kHandoffBytes / ((size_t)2 * H * 4));
   double best = 1e300;
-  for (int l = sc.variant ? 1 : 0; l < layouts(H); ++l) {
+  for (int l = 0; l < layouts(H); ++l) {
     const size_t ipw = (size_t)16 >> l;
     const size_t items = 2 * ((pl.chunk + ipw - 1) / ipw);
     const size_t cap = (size_t)resident_warps(H, l);

@@ -283,7 +283,7 @@ cudaError_t launch_sq_encrypt(int S, const KeyConst& kc, const EncArgs& a, uint3
   }
   int best = -1;
   double best_cost = 1e300;
-  for (int l = kc.variant ? 1 : 0; l < 5; ++l) {
+  for (int l = 0; l < 5; ++l) {
     if ((H != 32 && l == 0) || (H == 32 && l == 3)) continue;
     const size_t ipw = (size_t)16 >> l;
     const double per = std::ceil((double)((count + ipw - 1) / ipw) / scheds);

@@ -628,7 +628,7 @@ void core_inverse(KeyRec& k, Work& w, const uint32_t* in, const int64_t* sel, ui
 void mul_powers(KeyRec& k, Work& w, const uint32_t* a, const int64_t* kk, uint32_t* out, size_t count) {
   if (count == 0) return;
   if (k.kc.two_digit) {
-    const hg::MulPlan pl = hg::mul_plan(k.S, k.kc, count);
+    const hg::MulPlan pl = hg::mul_plan(k.S, count);
     uint32_t* scratch = w.scratch.ensure<uint32_t>(hg::mul_scratch_words(k.S, k.wm) * 4);
     cuda_check(hg::launch_sq_mul(k.S, k.kc, pl, a, kk, out, count, scratch, k.wm, w.errp(), w.ctrp(), w.stream),
                "mul launch");
@@ -2737,9 +2737,12 @@ int hg_autotune(hg_ctx* ctx, int key_id, size_t calib, hg_key_config* best, doub
       cudaEventElapsedTime(&ms, e0, e1);
       return (double)ms * 1e-3;
     };
+    // A two-digit key's layouts follow each call's length, so only its windows
+    // are compared: of one length's timings the variants would be noise.
     hg_key_config c = current_config(*k), bc = c;
+    const int v_first = k->kc.two_digit ? c.variant : 0, v_last = k->kc.two_digit ? c.variant : 1;
     double best_nn = 1e300, t_enc = 0, t_mul = 0;
-    for (int v = 0; v < 2; ++v) {
+    for (int v = v_first; v <= v_last; ++v) {
       c.variant = v;
       apply_config(*k, c);
       const double te = timed([&] { core_encrypt(*k, w, hg::EncMode::kEncrypt, dm, nullptr, nullptr, dr, nullptr, dct, n); });
@@ -2763,29 +2766,24 @@ int hg_autotune(hg_ctx* ctx, int key_id, size_t calib, hg_key_config* best, doub
     apply_config(*k, c);
     double t_dec = 0;
     if (k->secret) {
-      // fresh ciphertexts with the chosen variant
+      // fresh ciphertexts
       core_encrypt(*k, w, hg::EncMode::kEncrypt, dm, nullptr, nullptr, dr, nullptr, dct, n);
-      // enough ciphertexts for several waves of the widest layout, else the
-      // layout with more lanes per ciphertext wins on a half-empty GPU
+      // enough ciphertexts for several waves of the narrowest layout
       const size_t wave = hg::decrypt_wave(k->Sp);
       const size_t nd = std::min(n, std::max<size_t>(n / 2, 4 * wave));
       double best_d = 1e300;
-      for (int dv = 0; dv < 2; ++dv)
-        for (int wd = 4; wd <= 7; ++wd) {
-          c.dec_variant = dv;
-          c.dec_window = wd;
-          apply_config(*k, c);
-          const double td = timed([&] {
-            core_decrypt(*k, w, dct, dm2, reinterpret_cast<uint8_t*>(dm2 + nd), nullptr, nullptr, nd);
-          });
-          if (td < best_d) {
-            best_d = td;
-            bc.dec_variant = dv;
-            bc.dec_window = wd;
-          }
+      for (int wd = 4; wd <= hg::kMaxDecWindow; ++wd) {
+        c.dec_window = wd;
+        apply_config(*k, c);
+        const double td = timed([&] {
+          core_decrypt(*k, w, dct, dm2, reinterpret_cast<uint8_t*>(dm2 + nd), nullptr, nullptr, nd);
+        });
+        if (td < best_d) {
+          best_d = td;
+          bc.dec_window = wd;
         }
+      }
       t_dec = best_d / (double)nd;
-      c.dec_variant = bc.dec_variant;
       c.dec_window = bc.dec_window;
       apply_config(*k, c);
     }

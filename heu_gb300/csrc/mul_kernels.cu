@@ -76,7 +76,7 @@ int resident_warps(int H, int logtc) {
 
 }  // namespace
 
-MulPlan mul_plan(int S, const KeyConst& kc, size_t count) {
+MulPlan mul_plan(int S, size_t count) {
   const int H = S / 2;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -84,18 +84,20 @@ MulPlan mul_plan(int S, const KeyConst& kc, size_t count) {
   const double scheds = 4.0 * std::max(sms, 1);
   MulPlan pl;
   double best = 1e300;
-  bool first = true;
   for (int l = 1; l < 5; ++l) {
     if (!has_layout(H, l)) continue;
-    if (first && kc.variant) {  // variant 1 leaves out the narrowest layout
-      first = false;
-      continue;
-    }
-    first = false;
     const size_t ipw = (size_t)16 >> l;
     const size_t items = (count + ipw - 1) / ipw;
     const size_t cap = (size_t)resident_warps(H, l);
     const size_t rounds = (items + cap - 1) / cap;
+    // The pass costs are the encryption's; Mul's own products of two rows take
+    // (2, 32) at 2048 bits to 222 registers, two warps a scheduler.  A full round
+    // of it is the fastest all the same (9,728 scalars 2.69 ms against 2.84 with
+    // (4, 16), two rounds 4.87 against 4.98), but in a long column the four warps
+    // of (4, 16) cover for each other: 32,768 9.10 against 8.21, 2^20 253 against
+    // 233 (window 4).  1024 and 3072 bits keep their narrowest layout (2^17: 8.0 against
+    // 8.7, 66.1 against 68.4).
+    if (H == 64 && l == 1 && rounds > 2) continue;
     const size_t warps = (items + rounds - 1) / rounds;  // every warp the same number of items
     const double cost = (double)rounds * sq_pass_cost(H, l, std::ceil((double)warps / scheds));
     if (cost < best) {

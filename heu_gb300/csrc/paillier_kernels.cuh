@@ -32,7 +32,7 @@ struct KeyConst {
   int npos;             // digit positions = ceil(rbits / w)
   int rbits;            // bits of the encryption randomness r (k/2)
   int rlimbs;           // 32-bit limbs per r
-  int variant;          // (threads per instance, limbs per thread) variant, 0 or 1
+  int variant;          // 0 or 1: layout modulo n^2 of keys that are not two_digit, and of per-key batches
   // two-digit encryption (sq_encrypt.cuh; H = S/2 limbs of n, rho = 2^(32 (H+1))):
   // the table then holds entries (Y0 | y), Montgomery form of radix rho, those
   // of position 0 times 2^(32 S), the radix of the output
@@ -76,7 +76,7 @@ struct SecConst {
   int prog_len;             // both programs padded to this many steps
   int wd;                   // decryption window bits
   int Sp;                   // 32-bit limbs of p^2
-  int variant;              // 0, or 1: without the narrowest layout
+  int variant;              // 0 or 1: layout in per-key batches
 };
 
 // Okamoto-Uchiyama secret constants (ou/secret_key.h; decryptor.cc:27-45).
@@ -168,7 +168,7 @@ struct MulPlan {
   int logtc = 1;  // log2 of the lanes per chain
   int warps = 0;
 };
-MulPlan mul_plan(int S, const KeyConst& kc, size_t count);
+MulPlan mul_plan(int S, size_t count);
 size_t mul_scratch_words(int S, int wm);
 cudaError_t launch_sq_mul(int S, const KeyConst& kc, const MulPlan& pl, const uint32_t* a, const int64_t* k,
                           uint32_t* out, size_t count, uint32_t* scratch, int wm, uint32_t* err,
@@ -205,7 +205,7 @@ cudaError_t launch_decrypt(int Sp, const KeyConst& kc, const SecConst& sc, const
 int dec_latency_limbs(int H);  // limbs of 28 bits of a digit
 cudaError_t launch_dec_latency(int H, const KeyConst& kc, const SecConst& sc, const uint32_t* ct, size_t count,
                                uint32_t* z, uint32_t* err, cudaStream_t st);
-size_t decrypt_wave(int Sp);  // ciphertexts of one full wave of the widest layout
+size_t decrypt_wave(int Sp);  // ciphertexts of one full wave of the narrowest layout
 // OU decryption over S-limb ciphertexts with Sp-limb p^2 arithmetic
 // (S, Sp) in {(64, 32), (128, 64), (128, 96)}.
 cudaError_t launch_ou_decrypt(int S, const KeyConst& kc, const OuConst& oc, const uint32_t* ct, size_t count,

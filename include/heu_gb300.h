@@ -208,22 +208,25 @@ int hg_to_mont(hg_ctx* ctx, int key_id, const uint32_t* z, uint32_t* mont, size_
 int hg_from_mont(hg_ctx* ctx, int key_id, const uint32_t* mont, uint32_t* z, size_t count);
 
 /* ---- per-key tuning (no counterpart in the reference) --------------------
- * (threads per ciphertext, limbs per thread) variant and window widths.  The
- * results do not depend on the configuration, only the speed does.        */
+ * Window widths and layout variants.  The results do not depend on the
+ * configuration, only the speed does.  Calls choose their layout by their
+ * length; the variants are the layouts of HG_BATCH_PER_KEY batches, and
+ * `variant` also that of a key whose h_s shares a factor with n.            */
 typedef struct {
-  int variant;     /* mod n^2 ops: 0 = default layout, 1 = alternative */
-  int dec_variant; /* mod p^2 (CRT decryption): 0 or 1 */
-  int mul_window;  /* sliding-window bits of scalar Mul, 2..6 */
+  int variant;     /* encryption, Add and Mul: 0 or 1 */
+  int dec_variant; /* CRT decryption: 0 or 1 */
+  int mul_window;  /* window bits of scalar Mul, 2..6 */
   int dec_window;  /* sliding-window bits of CRT decryption, 2..7 */
 } hg_key_config;
 int hg_key_get_config(hg_ctx* ctx, int key_id, hg_key_config* out);
 int hg_key_set_config(hg_ctx* ctx, int key_id, const hg_key_config* cfg);
-/* Project autotuner: times encrypt and mul (both variants, mul windows 2..6)
- * and decrypt (both variants, windows 4..7) on `calib` random inputs
- * (0 = 65536; decryption uses enough of them for several full waves),
- * applies the fastest configuration and returns it; rates[0..2] receive
- * encrypt, mul and decrypt ops/s at that configuration.  Calibrate with at
- * least as many inputs as a production call fills the GPU with.          */
+/* Project autotuner: times encrypt and mul (mul windows 2..6) and decrypt
+ * (windows 4..7) on `calib` random inputs (0 = 65536; decryption uses enough
+ * of them for several full waves), applies the fastest windows and returns
+ * the configuration; rates[0..2] receive encrypt, mul and decrypt ops/s at
+ * that configuration.  The variants stay what they were, but for a key whose
+ * h_s shares a factor with n, where `variant` is compared too.  Calibrate
+ * with at least as many inputs as a production call fills the GPU with.   */
 int hg_autotune(hg_ctx* ctx, int key_id, size_t calib, hg_key_config* best, double* rates);
 
 /* ---- persistent multi-key batches (no counterpart in the reference) -----
@@ -250,7 +253,7 @@ int hg_batch_add(hg_batch* b, int key_id, int op, size_t count, const void* in0,
                  void* aux, int flags);
 int hg_batch_clear(hg_batch* b);
 /* Layout variant set of the batch's kernel: 0 or 1 for every job (default
- * 0), or HG_BATCH_PER_KEY: every job in its key's tuned layout
+ * 0), or HG_BATCH_PER_KEY: every job in the layout of its key
  * (hg_key_config: dec_variant for decryptions, variant for the other ops),
  * run as one persistent launch per variant set in use, back to back.    */
 #define HG_BATCH_PER_KEY (-1)

@@ -158,3 +158,21 @@ def test_a_short_call_leaves_room_for_a_long_one(gpu_key, bits, seed):
         g.replay()
         torch.cuda.synchronize()
         assert np.array_equal(out[:n].cpu().numpy(), m[:n]) and not out[n:].any()
+
+
+@pytest.mark.parametrize("bits,seed", [(1024, 1), (2048, 0), (3072, 2)])
+def test_the_tuner_chooses_windows_alone(gpu_key, bits, seed):
+    """Layouts follow the number of elements of each call, so one length's timing
+    must not take a layout away from the others: a key's layout variants are what
+    they were before."""
+    key, _, _ = gpu_key(bits, seed)
+    saved = autotune.get_config(key)
+    try:
+        for calib in (64, 300, 1000, 3000):
+            for variant in (0, 1):
+                autotune.set_config(key, dict(saved, variant=variant, dec_variant=variant))
+                cfg, rates = autotune.tune(key, calib=calib)
+                assert cfg["variant"] == variant and cfg["dec_variant"] == variant, calib
+                assert all(v > 0 for v in rates.values())
+    finally:
+        autotune.set_config(key, saved)
