@@ -18,6 +18,11 @@ from heu_gb300 import capi
 DEFAULT_CACHE = os.environ.get("HEU_GB300_TUNING",
                                os.path.join(os.path.expanduser("~"), ".cache", "heu_gb300", "tuning.json"))
 
+# Of the kernels that a configuration was tuned for: raised whenever one of its
+# values comes to select other code.  1 (not written): layouts modulo n^2 and p^2;
+# 2: two-digit arithmetic, Mul with windows at fixed places.
+REVISION = 2
+
 
 def device_name(device=0):
     try:
@@ -62,7 +67,7 @@ def save(config, key_bits, path=DEFAULT_CACHE, device=0, rates=None):
                     data = json.load(open(path))
                 except (OSError, ValueError):
                     data = {}
-            entry = {"config": config}
+            entry = {"config": config, "revision": REVISION}
             if rates:
                 entry["rates"] = rates
             data.setdefault(device_name(device), {})[str(key_bits)] = entry
@@ -76,9 +81,12 @@ def save(config, key_bits, path=DEFAULT_CACHE, device=0, rates=None):
 
 
 def load(key_bits, path=DEFAULT_CACHE, device=0):
+    """The recorded configuration, or None: also where it was tuned for other
+    kernels (REVISION)."""
     try:
         data = json.load(open(path))
-        return data[device_name(device)][str(key_bits)]["config"]
+        entry = data[device_name(device)][str(key_bits)]
+        return entry["config"] if entry.get("revision") == REVISION else None
     except (OSError, ValueError, KeyError):
         return None
 
