@@ -6,6 +6,7 @@
 #include "sqmod.cuh"
 
 namespace hg {
+inline namespace HG_SQ_SPACE {
 
 // m_p = z_p c1_p + c2_p mod p, the same for q, then the CRT combination
 //   h = (m_q - m_p) p^-1 mod q, m = m_p + p h
@@ -171,4 +172,5 @@ __device__ __forceinline__ void dec_pow_fixed(const KeyConst& kc, const SecConst
   }
 }
 
+}  // namespace HG_SQ_SPACE
 }  // namespace hg

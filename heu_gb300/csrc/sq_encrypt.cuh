@@ -16,6 +16,7 @@
 #include "sqmod.cuh"
 
 namespace hg {
+inline namespace HG_SQ_SPACE {
 
 // Shared words of a warp: two entries in flight and the sum of the y.
 template <int TC, int L>
@@ -249,4 +250,5 @@ __device__ __forceinline__ void sq_encrypt(const Mod& n, const KeyConst& kc, con
   if (active) store_slice<L>(out + i * S + g.c * H + g.t * L, r);
 }
 
+}  // namespace HG_SQ_SPACE
 }  // namespace hg

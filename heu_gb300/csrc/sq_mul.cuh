@@ -9,6 +9,7 @@
 #include "sqmod.cuh"
 
 namespace hg {
+inline namespace HG_SQ_SPACE {
 
 // `tb`: mul_slots(wm) entries of this warp, `area`: two digits.
 template <int TC, int L, class Mod>
@@ -75,4 +76,5 @@ __device__ __forceinline__ void sq_mul(const Mod& n, const KeyConst& kc, const u
   if (active) store_slice<L>(out + i * S + g.c * H + g.t * L, r);
 }
 
+}  // namespace HG_SQ_SPACE
 }  // namespace hg

@@ -30,7 +30,18 @@
 
 #include "mont.cuh"
 
+// Limbs a loop body of a pass takes (kSqUnroll); 0: by layout.  A unit that wants
+// another number (batch_v0.cu) gets its passes, and all that is built from them,
+// under names of their own.
+#ifndef HG_SQ_UNROLL
+#define HG_SQ_UNROLL 0
+#endif
+#define HG_SQ_JOIN_(a, b) a##b
+#define HG_SQ_JOIN(a, b) HG_SQ_JOIN_(a, b)
+#define HG_SQ_SPACE HG_SQ_JOIN(sq_unroll_, HG_SQ_UNROLL)
+
 namespace hg {
+inline namespace HG_SQ_SPACE {
 
 template <int TC, int L>
 struct SqLanes {
@@ -200,11 +211,7 @@ __device__ __forceinline__ void sq_settle(uint32_t (&x)[L], const uint32_t (&Ev)
 // limbs) 85.0, 81.9 and 80.5 ms, 65,536 of 2048 bits with 16 limbs a lane 97.4,
 // 91.0 and 87.7 ms.  (Multipliers in 16-byte loads then took 1 to 3% off each.)
 template <int TC, int L>
-#ifdef HG_SQ_UNROLL  // batch_v0.cu
-constexpr int kSqUnroll = HG_SQ_UNROLL;
-#else
-constexpr int kSqUnroll = TC == 1 && L == 32 ? 8 : 16;
-#endif
+constexpr int kSqUnroll = HG_SQ_UNROLL ? HG_SQ_UNROLL : TC == 1 && L == 32 ? 8 : 16;
 
 // Layouts whose passes run sq_step_early: the widest of the primes' lengths,
 // which only few ciphertexts take.  8 CRT decryptions of 2048 bits (16 lanes a
@@ -554,4 +561,5 @@ __device__ __forceinline__ void sq_to_raw(uint32_t (&r)[L], const uint32_t (&xin
   }
 }
 
+}  // namespace HG_SQ_SPACE
 }  // namespace hg
