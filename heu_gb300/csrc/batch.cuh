@@ -33,7 +33,7 @@ struct BatchTile {
 };
 
 // Lanes of an instance for n^2 with S limbs, and of a side of a decryption (two
-// chains) for p^2 with SP limbs, per variant; V = 2: the latency layout.
+// chains, one a digit) for p^2 of SP limbs, per variant; V = 2: the latency layout.
 __host__ __device__ constexpr int tpi_for(int S, int V) {
   return V == 2 ? 32 : S == 64 ? (V ? 8 : 4) : S == 128 ? (V ? 4 : 8) : (V ? 8 : 16);
 }

@@ -153,10 +153,11 @@ __global__ void __launch_bounds__(batch_detail::kBlock, V == 1 ? 1 : 4) k_batch(
   uint32_t* ws = scratch + ((size_t)blockIdx.x * batch_detail::kWarps + wib) * warp_words;
   // The first claims go round the chip, one warp a block: warp 1 waits 2 us, warp
   // 2 four and warp 3 six, while the launch's blocks arrive.  Without that the
-  // multiprocessors whose blocks arrived first took the long chains four to a
-  // scheduler: 1,025 decryptions of 3072 bits alone 24.8 ms against 10.1, 4,096
-  // of 2048 bits 14.5 against 8.5, a mixed batch of 47,452 operations 30.6
-  // against 24.1 (19.3 against 21.0 with the next batch queued behind it).
+  // multiprocessors whose blocks arrived first take the chains four to a
+  // scheduler.  1,025 decryptions of 3072 bits alone: 10.1 ms with the wait, 27.3
+  // without, 4,096 of 2048 bits 8.4 and 16.6, 600 additions of 2048 bits 0.076 and
+  // 0.104, one addition 0.031 and 0.032; a mixed batch of 47,452 operations 24.0
+  // and 28.3, and 19.2 and 18.9 with the next batch queued behind it.
   const long long started = clock64();
   while (clock64() - started < (long long)wib * batch_detail::kFirstClaimCycles) {
   }

@@ -82,10 +82,11 @@ __device__ __forceinline__ void dec_pow_side(const Mod& n, const KeyConst& kc, c
   if (active && g.c == 1) store_slice<L>(z + (2 * i + side) * H + g.t * L, x);
 }
 
-// Resident warps per SM that the compiler must fit, one warp per block.  The
-// multiply-add pipe is 91% busy at 8 warps, so the one-lane layouts take the
-// registers they need: 65,536 decryptions of 2048 bits took 89.8 ms at 10 warps
-// against 92.0 at 12 and 100.7 at 16, whose two-row pass spills.
+// Resident warps per SM that the compiler must fit, one warp per block.  With 32
+// limbs a lane 9 to 12 are the same three warps a scheduler: 168 registers, 396
+// bytes of spills.  8 take 234 registers and none: 2^20 decryptions of 2048 bits
+// 1,328 ms against 1,267 at 12, 65,536 88.1 against 86.8, but 14,592 (one round
+// of 12) 20.3 against 21.0 and 29,184 38.5 against 42.9.
 constexpr int dec_min_blocks(int L) { return L == 48 ? 8 : L == 32 ? 10 : L == 24 ? 12 : L == 16 ? 16 : L == 12 ? 18 : 20; }
 
 // One warp per block: warps take (side, group of instances) items from the

@@ -224,8 +224,10 @@ __global__ void __launch_bounds__(128) k_sq_level(const __grid_constant__ KeyCon
 }  // namespace
 
 // Time per product of one warp (us) when every scheduler holds `warps` warps of
-// a layout, as measured on GB300: few ciphertexts run fastest with many lanes a
-// chain, many with few.  2048 bits, window 12: 608 ciphertexts take 0.31 ms
+// a layout, as measured on GB300 with encryption's passes of one row (Mul and
+// MatMul, which also choose by it, run passes of two as well and hold other
+// numbers of registers): few ciphertexts run fastest with many lanes a chain,
+// many with few.  2048 bits, window 12: 608 ciphertexts take 0.31 ms
 // with 16 lanes a chain (0.67 with 4), 4,864 take 0.99 ms with 4 (1.25 with 2
 // or 16), 131,072 take 23.5 ms with 2, 23.9 with 4 and 30.9 with 16.
 double sq_pass_cost(int H, int logtc, double warps) {
@@ -303,8 +305,6 @@ cudaError_t launch_sq_encrypt(int S, const KeyConst& kc, const EncArgs& a, uint3
   count_launches(1);
   return cudaGetLastError();
 }
-
-size_t sq_base_words(int S, int npos) { return (size_t)npos * 3 * (S / 2); }
 
 cudaError_t launch_sq_bases(int S, const KeyConst& kc, const uint32_t* first, uint32_t* bases, cudaStream_t st) {
   HG_DISPATCH_SQ16(S / 2, k_sq_bases<TC, L><<<1, 64, 0, st>>>(kc, first, bases));

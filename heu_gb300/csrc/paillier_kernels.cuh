@@ -173,8 +173,8 @@ size_t mul_scratch_words(int S, int wm);
 cudaError_t launch_sq_mul(int S, const KeyConst& kc, const MulPlan& pl, const uint32_t* a, const int64_t* k,
                           uint32_t* out, size_t count, uint32_t* scratch, int wm, uint32_t* err,
                           unsigned long long* ctr, cudaStream_t st);
-// Time (us) of a pass modulo an H-limb n's square with `warps` warps of a
-// layout on every scheduler (encrypt_kernels.cu).
+// Time (us) of an encryption's pass modulo an H-limb n's square with `warps`
+// warps of a layout on every scheduler (encrypt_kernels.cu).
 double sq_pass_cost(int H, int logtc, double warps);
 // Mul by multi-limb scalar magnitudes (el limbs each), window wb (1..8);
 // persistent grid of `grid` blocks (resident_blocks_mul_bn) with a scratch of

@@ -366,8 +366,8 @@ void finish_req(hg_server& s, Req* q) {
 
 // Class of a pending request: 0 regular, 1 express, 2 slow express.
 // With express_len, short = at most express_len elements; short CRT
-// decryptions (a chain of ~2,400 dependent Montgomery steps, several ms even
-// on an idle GPU) get the second express slot when there is one, so a batch
+// decryptions (a chain of about 1,250 dependent products at 2048 bits, several
+// ms even on an idle GPU) get the second express slot when there is one, so a batch
 // of the other short ops never waits for them.  Without express_len, short
 // = estimated remaining work <= express_us.
 int req_class(const hg_server& s, const Req* q) {

@@ -333,9 +333,14 @@ __global__ void __launch_bounds__(32) k_mm_planes(const __grid_constant__ KeyCon
     default: return cudaErrorInvalidValue;                                      \
   }
 
-// Nodes of a level up to which the widest layout is as fast: its warps take
-// one product each, a few per SM.
-constexpr size_t kWideNodes = 2432;
+// Nodes of a level up to which the widest layout is as fast: its warps take two
+// products each, 8 per SM.
+size_t wide_nodes() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return (size_t)16 * std::max(sms, 1);
+}
 
 template <int TC, int L>
 unsigned pair_blocks(size_t count) {
@@ -385,7 +390,7 @@ cudaError_t launch_mm_log(int S, const KeyConst& kc, size_t rows, int K, int b, 
 cudaError_t launch_half_up(int S, const KeyConst& kc, const uint32_t* lower, size_t lower_count, uint32_t* upper,
                            cudaStream_t st) {
   const size_t total = (lower_count + 1) / 2;
-  if (total <= kWideNodes) {
+  if (total <= wide_nodes()) {
     HG_DISPATCH_MM16(S / 2,
                      k_half_up<TC, L><<<pair_blocks<TC, L>(total), 128, 0, st>>>(kc, lower, lower_count, upper));
   } else {
@@ -399,7 +404,7 @@ cudaError_t launch_half_up(int S, const KeyConst& kc, const uint32_t* lower, siz
 cudaError_t launch_half_down(int S, const KeyConst& kc, uint32_t* lower, size_t lower_count, const uint32_t* upper,
                              cudaStream_t st) {
   const size_t total = (lower_count + 1) / 2;
-  if (total <= kWideNodes) {
+  if (total <= wide_nodes()) {
     HG_DISPATCH_MM16(S / 2,
                      k_half_down<TC, L><<<pair_blocks<TC, L>(total), 128, 0, st>>>(kc, lower, lower_count, upper));
   } else {

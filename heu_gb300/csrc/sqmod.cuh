@@ -229,8 +229,11 @@ constexpr bool kSqEarly = L == 2 || (TC == 8 && L == 6);
 //   product with Y:   x = Y's digit of the chain, y = X0, x2 = Y0, y2 = X1 (chain 1)
 //   times integer Y0: x = Y0, y = own digit of X
 // kJoin = false: z_c = x_c * y_c / rho modulo n in each chain for itself.
-// `ytop` is limb H of an undoubled multiplier (a few units: the result's
-// bound holds).
+// `ytop` is limb H of an undoubled multiplier: below 2^31 it leaves the result
+// below n + x / 2, so the subtraction behind the vote brings it below 2^(32 H)
+// and the caller's one more, x being less than 2 n, below n.  The encryption's is
+// the top word of a sum of npos + 2 numbers, MatMul's that of its doubled sum,
+// which launch_mm_planes holds below 2^31.
 template <int TC, int L, bool kTwo, bool kJoin = true, class Mod>
 __device__ __forceinline__ void sq_pass(uint32_t (&z)[L], const uint32_t (&x)[L], const uint32_t* y, uint32_t dbl,
                                         uint32_t ytop, const uint32_t (&x2)[L], const uint32_t* y2, const Mod& n,
