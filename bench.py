@@ -101,6 +101,14 @@ def mul_macs_mont(key_bits, ks, wm=4):
 
 
 # ---------------------------------------------------------------------------
+def imad_peak(sms, clocks):
+    """TMAC/s that the fmaheavy pipe can issue: a wide 32x32->64 multiply-add every 4
+    cycles of a sub-partition, 32 a clock an SM, at the SM clock sampled under load
+    (the maximum where none was).  None without a clock."""
+    mhz = (clocks or {}).get("sm_mhz") or (clocks or {}).get("sm_max_mhz")
+    return 32 * sms * mhz / 1e6 if mhz else None
+
+
 class ClockSampler:
     """nvidia-smi clocks and throttle reasons sampled every 200 ms."""
 
@@ -454,14 +462,12 @@ def ours_arm(args):
         torch.cuda.synchronize()
         per_op["mul_nonneg_k"] = n * args.steps / (ea.elapsed_time(eb) / 1e3)
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    mhz = (clocks or {}).get("sm_mhz") or (clocks or {}).get("sm_max_mhz")
-    issue_bound = 32 * sms * mhz * 1e6 / 1e12 if mhz else None
+    peak = imad_peak(sms, clocks)
     macs_dec = decrypt_macs(KEY_BITS) * n
     dec_avg = op_s["decrypt"] / args.steps
     achieved = macs_dec / dec_avg / 1e12 if "decrypt" in ops else None
     peak_chain = capi.mac_peak(local, 0) / 1e12
     peak_wide = capi.mac_peak(local, 1) / 1e12
-    peak = max(peak_chain, peak_wide)
     k_host = kk.cpu().numpy()
     work = {
         "encrypt": encrypt_macs(KEY_BITS, args.window) * n,
@@ -614,15 +620,13 @@ def ours_arm(args):
                             "mul work in two digits to the base of the modulus' root, the CPU restatement modulo "
                             "the square"),
             "roofline": {"bound": "imad", "kernel": "decrypt (CRT, k_dec_pow)", "achieved": achieved,
-                         "peak": peak, "unit": "TMAC/s", "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                         "peak_source": "measured live: hg_probe_mac_peak (best of mad.wide / carry-chain "
-                                        "patterns); MEASURED_PEAKS.json has no integer figure",
-                         "peak_chain_pattern": peak_chain, "peak_wide_pattern": peak_wide,
-                         # the issue bound of the wide multiply-add: 4 cycles per warp
-                         # instruction on each SM sub-partition's fmaheavy pipe = 32 MACs per
-                         # clock per SM, at the SM clock sampled during the timed region
-                         "issue_bound": issue_bound, "frac_of_issue_bound": (achieved / issue_bound)
-                         if (achieved and issue_bound) else None,
+                         "peak": peak, "unit": "TMAC/s", "frac": (achieved / peak) if (achieved and peak) else None,
+                         "traffic": traffic,
+                         "peak_source": "issue bound of the wide multiply-add, 32 a clock an SM at the SM clock "
+                                        "sampled under load; MEASURED_PEAKS.json has no integer figure",
+                         # loops of other multiply-add forms (hg_probe_mac_peak), for comparison: the
+                         # kernels' paired rows run above both
+                         "probe_chain_pattern": peak_chain, "probe_wide_pattern": peak_wide,
                          "per_op_tmacs": roof_ops},
             "parity_checked": parity_checked,
             "parity": ("strided sample of the timed Encrypt / Add / Mul outputs byte-equal (Montgomery form) to "
@@ -915,7 +919,6 @@ def c3_measure(args, steps, warmup):
     if "matmul" in res:
         dm, _ = key_dec(mm)
         assert np.array_equal(dm.reshape(M, N), gh[: M * K].reshape(M, K) @ y)
-    peak = max(capi.mac_peak(0, 0), capi.mac_peak(0, 1)) / 1e12
     line = {
         "metric": "heu.numpy reductions on 2048-bit ciphertexts (config 3): Sum, bucket-sum, MatMul",
         "value": res[next(iter(res))]["units_per_s"] if "bucket_sum" not in res else res["bucket_sum"]["units_per_s"],
@@ -923,7 +926,7 @@ def c3_measure(args, steps, warmup):
         "n_gpus": 1, "steps": steps, "warmup": warmup, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "u32", "data": "synthetic",
         "config": {"workload": "config3", "sum_n": n, "bucket_sum": [n, F, B], "matmul": [M, K, N]},
-        "results": res, "mac_peak_tmacs": peak,
+        "results": res,
     }
     ctx.close()
     return line
@@ -1007,7 +1010,7 @@ def ou_arm(args):
         "mul": mul_macs_mont(2048, kk[: 1 << 14].cpu().numpy()) * (n / min(n, 1 << 14)),
         "decrypt": ((t_bits - 1) + -(-t_bits // (wd + 1)) + 2 ** (wd - 1) + 3) * mm_macs(64) * n,
     }
-    peak = max(capi.mac_peak(0, 0), capi.mac_peak(0, 1)) / 1e12
+    peak = imad_peak(ctx.sm_count(), clocks)
     tmacs = {nm: work[nm] / op_s[nm] / 1e12 for nm in names}
     # the OU oracle on one host core, bounded sample
     from oracle import ou
@@ -1044,7 +1047,7 @@ def ou_arm(args):
                    "table_window": w, "ciphertext_limbs": S},
         "per_op_ops_per_s": {nm: n / op_s[nm] for nm in names},
         "roofline": {"bound": "imad", "unit": "TMAC/s", "per_op_tmacs": tmacs, "peak": peak,
-                     "frac": {nm: tmacs[nm] / peak for nm in names}},
+                     "frac": {nm: tmacs[nm] / peak if peak else None for nm in names}},
         "cpu_baseline": {"value": cpu_rate, "unit": UNIT, "cores": 1, "kind": "port", "per_op": rates,
                          "sample": f"OU oracle (Python integers), {ns} enc/add, 100 mul, 200 dec, one core"},
         "clocks": clocks,

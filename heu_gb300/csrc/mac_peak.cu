@@ -1,5 +1,7 @@
-// Integer multiply-accumulate throughput probe (the roofline denominator for
-// the Montgomery kernels).  Pure register work, no memory traffic:
+// Integer multiply-accumulate throughput probe, for comparison with the kernels:
+// their paired rows (mont.cuh) issue one wide multiply-add a product with its
+// carry and run above both patterns; the bound is the pipe's issue rate, 32 a
+// clock an SM.  Pure register work, no memory traffic:
 //   pattern 0: 32x32->64 MACs as carry chains of mad.lo.cc / madc.hi.cc
 //              (2 instructions per MAC);
 //   pattern 1: 32x32->64 MACs as mad.wide.u32 into 64-bit accumulators.
