@@ -227,13 +227,11 @@ DecryptPlan decrypt_plan(int Sp, const SecConst& sc, size_t count) {
   pl.latency = count <= (size_t)std::max(sms, 1);
   const size_t slots = ((size_t)1 << (sc.wd - 1)) + 1;
   pl.table_words = pl.latency ? 0 : (size_t)pl.warps * slots * 32 * (size_t)(H >> pl.logtc);
+  pl.handoff_words = pl.chunk * 2 * (size_t)H;
   return pl;
 }
 
-// The most that any count's plan takes.  A stream's buffer has this size from its
-// first call on: a longer call then neither allocates (which a capture forbids)
-// nor frees a buffer that a captured graph still names.  2048 bits at window 6:
-// 363 MiB, a new stream's first call 0.11 ms longer than with 8 ciphertexts' own.
+// The most that any count's plan takes.
 size_t decrypt_scratch_words(int Sp, const SecConst& sc) {
   const int H = Sp / 2;
   const size_t slots = ((size_t)1 << (sc.wd - 1)) + 1;

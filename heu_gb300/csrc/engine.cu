@@ -120,7 +120,12 @@ struct DevBuf {
       }
       p = nullptr;
       n = 0;
-      cuda_check(cudaMalloc(&p, bytes), "cudaMalloc");
+      // the first allocation of a buffer may fall into the capture of a stream
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      const cudaError_t e = cudaMalloc(&p, bytes);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      cuda_check(e, "cudaMalloc");
       n = bytes;
       g_dev_bytes += n;
     }
@@ -268,6 +273,17 @@ struct Work {
   InvTask task;
   ~Work() {
     if (own_stream && stream) cudaStreamDestroy(stream);
+  }
+  // Scratch of a call that takes `words`, of a route whose longest calls take
+  // `most`: neither buffer grows with the length of the calls, so what a captured
+  // graph names stays.  A stream of short calls alone takes the runtime's piece of a
+  // 2 MiB block: a new one's first decryption of 8 takes 1.03 ms, 1.16 from 4 MiB up
+  // (long ones take 363 MiB at 2048 bits).
+  static constexpr size_t kSmallScratch = (size_t)256 << 10;
+  DevBuf small;
+  uint32_t* scratch_for(size_t words, size_t most) {
+    if (words * 4 <= kSmallScratch) return small.ensure<uint32_t>(kSmallScratch);
+    return scratch.ensure<uint32_t>(most * 4);
   }
   DevBuf ctr;  // work counter of the persistent kernels this lane launches
   uint32_t* errp() { return err.ensure<uint32_t>(sizeof(uint32_t)); }
@@ -505,7 +521,7 @@ void decrypt_crt(KeyRec& k, Work& w, const uint32_t* ct, int64_t* m, uint8_t* ov
   if (!k.secret) fail(HG_ERR_NO_SECRET, "key has no secret part");
   if (count == 0) return;
   const hg::DecryptPlan pl = hg::decrypt_plan(k.Sp, k.sc, count);
-  uint32_t* scratch = w.scratch.ensure<uint32_t>(hg::decrypt_scratch_words(k.Sp, k.sc) * 4);
+  uint32_t* scratch = w.scratch_for(pl.table_words + pl.handoff_words, hg::decrypt_scratch_words(k.Sp, k.sc));
   cuda_check(hg::launch_decrypt(k.Sp, k.kc, k.sc, k.primes.data(), pl, ct, count, m, ovf, mag, neg, scratch, w.errp(),
                                 w.ctrp(), w.stream, cd),
              "decrypt launch");
@@ -628,8 +644,8 @@ void core_inverse(KeyRec& k, Work& w, const uint32_t* in, const int64_t* sel, ui
 void mul_powers(KeyRec& k, Work& w, const uint32_t* a, const int64_t* kk, uint32_t* out, size_t count) {
   if (count == 0) return;
   if (k.kc.two_digit) {
-    const hg::MulPlan pl = hg::mul_plan(k.S, count);
-    uint32_t* scratch = w.scratch.ensure<uint32_t>(hg::mul_scratch_words(k.S, k.wm) * 4);
+    const hg::MulPlan pl = hg::mul_plan(k.S, k.wm, count);
+    uint32_t* scratch = w.scratch_for(pl.scratch_words, hg::mul_scratch_words(k.S, k.wm));
     cuda_check(hg::launch_sq_mul(k.S, k.kc, pl, a, kk, out, count, scratch, k.wm, w.errp(), w.ctrp(), w.stream),
                "mul launch");
     return;

@@ -76,7 +76,7 @@ int resident_warps(int H, int logtc) {
 
 }  // namespace
 
-MulPlan mul_plan(int S, size_t count) {
+MulPlan mul_plan(int S, int wm, size_t count) {
   const int H = S / 2;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -106,10 +106,11 @@ MulPlan mul_plan(int S, size_t count) {
       pl.warps = (int)warps;
     }
   }
+  pl.scratch_words = (size_t)pl.warps * mul_slots(wm) * 32 * (size_t)(H >> pl.logtc);
   return pl;
 }
 
-// The most that any count's plan takes, as decrypt_scratch_words.
+// The most that any count's plan takes.
 size_t mul_scratch_words(int S, int wm) {
   const int H = S / 2;
   size_t words = 0;

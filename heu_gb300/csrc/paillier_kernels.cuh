@@ -162,13 +162,14 @@ cudaError_t launch_add_plain(int S, const KeyConst& kc, const uint32_t* a, const
 cudaError_t launch_mul(int S, const KeyConst& kc, const uint32_t* a, const int64_t* k, uint32_t* out,
                        size_t count, uint32_t* scratch, int wm, uint32_t* err, int grid, unsigned long long* ctr,
                        cudaStream_t st);
-// Mul of two-digit keys (mul_kernels.cu); `scratch` holds mul_scratch_words
-// limbs.
+// Mul of two-digit keys (mul_kernels.cu) over mul_plan's scratch, which is
+// mul_scratch_words at most.
 struct MulPlan {
   int logtc = 1;  // log2 of the lanes per chain
   int warps = 0;
+  size_t scratch_words = 0;
 };
-MulPlan mul_plan(int S, size_t count);
+MulPlan mul_plan(int S, int wm, size_t count);
 size_t mul_scratch_words(int S, int wm);
 cudaError_t launch_sq_mul(int S, const KeyConst& kc, const MulPlan& pl, const uint32_t* a, const int64_t* k,
                           uint32_t* out, size_t count, uint32_t* scratch, int wm, uint32_t* err,
@@ -187,14 +188,14 @@ int resident_blocks_mul_bn(int S);
 cudaError_t launch_sel_from_neg(const uint8_t* neg, int64_t* sel, size_t count, cudaStream_t st);
 // With cd.kind != kCodecNone out_i64 receives the decoded values (int64 or
 // double, per cd.kind) and cd.out1 the second slot of batch kinds.
-// `primes`: p and q on the host (Sp/2 limbs each); `scratch` holds
-// decrypt_scratch_words limbs.
+// `primes`: p and q on the host (Sp/2 limbs each); `scratch` holds decrypt_plan's
+// table_words + handoff_words limbs, decrypt_scratch_words at most.
 struct DecryptPlan {
   bool latency = false;  // few ciphertexts: decrypt_latency.cu
   int logtc = 0;         // log2 of the lanes per chain
   int warps = 0;         // warps of the exponentiation launch
   size_t chunk = 0;      // ciphertexts per pair of launches
-  size_t table_words = 0;  // of the scratch, before the digits handed over
+  size_t table_words = 0, handoff_words = 0;
 };
 DecryptPlan decrypt_plan(int Sp, const SecConst& sc, size_t count);
 size_t decrypt_scratch_words(int Sp, const SecConst& sc);

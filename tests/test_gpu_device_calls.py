@@ -1,6 +1,6 @@
 """What a device call asks of its caller besides its values: the alignment of
-its arrays, that calls of other threads and keys leave it alone, and what a
-first call allocates."""
+its arrays, that calls of other threads and keys leave it alone, and what its
+stream allocates."""
 
 import ctypes
 import threading
@@ -111,11 +111,11 @@ def _held(lib):
 
 
 @pytest.mark.parametrize("bits,seed", [(1024, 1), (2048, 0), (3072, 2)])
-def test_a_short_call_leaves_room_for_a_long_one(gpu_key, bits, seed):
-    """A stream's first decryption allocates what one of any length takes, and
-    its first Mul all but the batch inverse's tree: a longer decryption after a
-    short one neither allocates nor frees, so it may be captured, and what was
-    captured before it stays valid."""
+def test_scratch_does_not_follow_the_length_of_the_calls(gpu_key, bits, seed):
+    """A stream allocates for decryptions (and all but the inverse's tree for
+    Muls) twice at most, once for short and once for any longer calls, and frees
+    nothing: a long call may be captured after a short one, and what was captured
+    before a longer call stays valid."""
     dev = torch.device("cuda", 0)
     key, _, _ = gpu_key(bits, seed)
     lib, h = key.lib, key.ctx.handle
@@ -125,32 +125,43 @@ def test_a_short_call_leaves_room_for_a_long_one(gpu_key, bits, seed):
     ct = torch.empty((count, key.ct_limbs), dtype=torch.int32, device=dev)
     prod, ones = torch.empty_like(ct), torch.ones(count, dtype=torch.int64, device=dev)
     out, ovf = torch.zeros(count, dtype=torch.int64, device=dev), torch.empty(count, dtype=torch.uint8, device=dev)
-    stream, other = torch.cuda.Stream(), torch.cuda.Stream()
-    s, s2 = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p(other.cuda_stream)
+    streams = [torch.cuda.Stream() for _ in range(3)]
     torch.cuda.synchronize()
-    capi.check(lib.hg_dev_encrypt(h, key.id, _p(dm), _p(dr), _p(ct), count, s))
+    capi.check(lib.hg_dev_encrypt(h, key.id, _p(dm), _p(dr), _p(ct), count, None))
     torch.cuda.synchronize()
 
-    def decrypt(n):
+    def decrypt(n, stream):
+        s = ctypes.c_void_p(stream.cuda_stream)
         capi.check(lib.hg_dev_decrypt(h, key.id, _p(ct), _p(out), _p(ovf), n, s))
 
-    decrypt(1)
+    def mul(n, stream):
+        s = ctypes.c_void_p(stream.cuda_stream)
+        capi.check(lib.hg_dev_mul(h, key.id, _p(ct), _p(ones), _p(prod), n, s))
+
+    decrypt(1, streams[0])
     base = _held(lib)
-    for n in (2, 700, 2500, count):
-        decrypt(n)
+    for n in (2, 3, 7):
+        decrypt(n, streams[0])
         assert _held(lib) == base, n
-    capi.check(lib.hg_dev_mul(h, key.id, _p(ct), _p(ones), _p(prod), 3, s2))
+    decrypt(2500, streams[0])
     base = _held(lib)
-    capi.check(lib.hg_dev_mul(h, key.id, _p(ct), _p(ones), _p(prod), count, s2))
+    for n in (5, 700, 3000, count // 2, count):
+        decrypt(n, streams[0])
+        assert _held(lib) == base, n
+    mul(2500, streams[1])
+    base = _held(lib)
+    mul(count, streams[1])
     tree = (2 * count + 64) * key.ct_limbs * 4
     assert base <= _held(lib) <= base + tree
     torch.cuda.synchronize()
     assert torch.equal(prod, ct)
+    # a stream that has seen one short call; the short graph runs after the long one
+    decrypt(1, streams[2])
     graphs = []
     for n in (5, count):
         g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g, stream=stream):
-            decrypt(n)
+        with torch.cuda.graph(g, stream=streams[2]):
+            decrypt(n, streams[2])
         graphs.append((n, g))
     for n, g in graphs[::-1]:
         out.zero_()
